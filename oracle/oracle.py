@@ -32,11 +32,11 @@ _lib = None
 
 def build(force: bool = False, reference: str | None = None) -> None:
     """Compile liboracle.so, and oracle/_ref from the reference source tree at `reference`
-    (default: the GZ_REFERENCE environment variable) when that tree exists."""
+    (default: the GZ_REFERENCE environment variable) when that tree holds its sources."""
     targets = ["oracle"]
     ref = reference or os.environ.get("GZ_REFERENCE", "")
     env = dict(os.environ)
-    if ref and os.path.isdir(ref):
+    if ref and os.path.isfile(os.path.join(ref, "src", "sketch.cpp")):
         targets.append("ref")
         env["REF"] = ref
     args = ["make", "-C", HERE] + (["-B"] if force else []) + targets
