@@ -181,11 +181,12 @@ struct gz_alg {
   bool eager = false, host_answer = false, boruvka_ran = false;
   std::vector<uint32_t> hdsu;
   std::unordered_set<uint64_t> hforest;
-  // how a query runs: 2 = one cooperative kernel (every round on the device), 1 = a CUDA graph of
+  // how a query runs: 2 = one kernel launch (every round on the device), 1 = a CUDA graph of
   // the per-phase kernels with a conditional while node over the rounds (qgraph), 0 = the same
   // kernels with the round loop on the host, -1 = by size (query_mode_of)
   gz::BoruvkaGraph qgraph;
   int query_mode = -1;
+  bool no_one_launch = false;  // the one-launch query's buffers could not be allocated
   uint32_t *h_qpin = nullptr;  // pinned: rounds, out-of-samples flag, components
   // queries by ticket (gz_query_submit / gz_query_wait): the query graph enqueued on the
   // handle's stream behind every update submitted before it, with its own buffers, so the
@@ -561,37 +562,7 @@ void destroy_alg(gz_alg *h) {
     if (h->ev_ent_done[i]) cudaEventDestroy(h->ev_ent_done[i]);
   }
   dev_free(h->d_raw);
-  auto &b = h->bv;
-  dev_free(b.parent);
-  dev_free(b.label);
-  dev_free(b.cnt);
-  dev_free(b.fill);
-  dev_free(b.minv);
-  dev_free(b.packed);
-  dev_free(b.scan_total);
-  dev_free(b.scan_tmp);
-  dev_free(b.order);
-  dev_free(b.order_comp);
-  dev_free(b.comp_start);
-  dev_free(b.comp_key);
-  dev_free(b.ncomp);
-  dev_free(b.acc);
-  dev_free(b.part);
-  dev_free(b.part_comp);
-  dev_free(b.big);
-  dev_free(b.round);
-  b.ctl = nullptr;
-  dev_free(b.flags);
-  dev_free(b.cross);
-  dev_free(b.ncross);
-  dev_free(b.qbar);
-  dev_free(b.btot);
-  dev_free(b.forest);
-  dev_free(b.forest_n);
-  if (b.trace) cudaFree(b.trace);
-  dev_free(b.trace_n);
-  dev_free(h->d_final);
-  dev_free(h->d_ncc);
+  free_bv(h->bv);
   for (auto &e : h->prof_pending) {
     cudaEventDestroy(e.a);
     cudaEventDestroy(e.b);
@@ -836,6 +807,7 @@ int eager_from_device(gz_alg *h, bool have_forest) {
     if (n) GZ_CUDA(cudaMemcpyAsync(idx.data(), h->bv.forest, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
   }
   GZ_CUDA(cudaStreamSynchronize(h->stream));
+  idx.erase(std::remove(idx.begin(), idx.end(), gz::kNoEdge), idx.end());
   h->hforest.clear();
   h->hforest.insert(idx.begin(), idx.end());
   h->host_answer = false;
@@ -844,88 +816,121 @@ int eager_from_device(gz_alg *h, bool have_forest) {
 
 // ---- Boruvka ---------------------------------------------------------------------------------------
 
-// Boruvka buffers for V vertices; acc_words per component spanning warps (and per merge warp)
-int alloc_bv(gz::BoruvkaBufs &b, size_t V, size_t acc_words, uint32_t *status) {
-  GZ_TRY(dev_alloc(&b.parent, V));
-  GZ_TRY(dev_alloc(&b.label, V));
-  GZ_TRY(dev_alloc(&b.cnt, V));
-  GZ_TRY(dev_alloc(&b.fill, V));
-  GZ_TRY(dev_alloc(&b.minv, V));
-  GZ_TRY(dev_alloc(&b.packed, V));
-  GZ_TRY(dev_alloc(&b.scan_total, 1));
-  GZ_TRY(dev_alloc(&b.scan_tmp, gz::scan_tmp_words(V)));
-  GZ_TRY(dev_alloc(&b.order, V));
-  GZ_TRY(dev_alloc(&b.order_comp, V));
-  GZ_TRY(dev_alloc(&b.comp_start, V + 1));
-  GZ_TRY(dev_alloc(&b.comp_key, V));
-  GZ_TRY(dev_alloc(&b.ncomp, 1));
-  const size_t warps = (V + gz::kBoruvkaSpan - 1) / gz::kBoruvkaSpan;
-  GZ_TRY(dev_alloc(&b.acc, (warps + 1) * acc_words));
-  GZ_TRY(dev_alloc(&b.part, warps * acc_words));
-  GZ_TRY(dev_alloc(&b.part_comp, warps));
-  GZ_TRY(dev_alloc(&b.big, 1));
-  GZ_TRY(dev_alloc(&b.round, 4));
+// One device allocation cut into 256-byte aligned arrays (a handle's first query would otherwise pay
+// for some twenty cudaMalloc calls): each take() notes where an array goes, alloc() makes the block
+// and sets the pointers.
+struct Block {
+  struct Part {
+    void **p;
+    size_t off;
+  };
+  std::vector<Part> parts;
+  size_t bytes = 0;
+  template <class T>
+  void take(T **p, size_t count) {
+    parts.push_back({reinterpret_cast<void **>(p), bytes});
+    bytes += (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+  }
+  int alloc(uint8_t **base) {
+    GZ_TRY(dev_alloc(base, bytes));
+    for (const Part &x : parts) *x.p = *base + x.off;
+    return GZ_OK;
+  }
+};
+
+// Boruvka buffers for V vertices that every query mode uses.
+int alloc_bv(gz::BoruvkaBufs &b, size_t V, uint32_t *status, uint32_t **labels, uint32_t **ncc) {
+  if (b.block) return GZ_OK;
+  Block k;
+  k.take(&b.parent, V);
+  k.take(&b.label, V);
+  k.take(&b.minv, V);
+  k.take(&b.forest, V);
+  k.take(labels, V);
+  k.take(&b.round, 8);  // round, ctl[3], components
+  k.take(&b.flags, 4);
+  k.take(&b.forest_n, 1);
+  k.take(&b.trace_n, 1);
+  GZ_TRY(k.alloc(&b.block));
   b.ctl = b.round + 1;
-  GZ_TRY(dev_alloc(&b.flags, 4));
-  GZ_TRY(dev_alloc(&b.cross, warps + 1));
-  GZ_TRY(dev_alloc(&b.ncross, 1));
-  GZ_TRY(dev_alloc(&b.qbar, 1));
-  GZ_TRY(dev_alloc(&b.btot, gz::kBvQueryMaxBlocks));
-  GZ_TRY(dev_alloc(&b.forest, V));
-  GZ_TRY(dev_alloc(&b.forest_n, 1));
-  GZ_TRY(dev_alloc(&b.trace_n, 1));
+  *ncc = b.round + 4;
   b.status = status;
   return GZ_OK;
 }
 
+// Those of the per-phase kernels (query modes 0 and 1); acc_words per component spanning warps (and
+// per merge warp).
+int alloc_bv_phases(gz::BoruvkaBufs &b, size_t V, size_t acc_words) {
+  if (b.block_phases) return GZ_OK;
+  const size_t warps = (V + gz::kBoruvkaSpan - 1) / gz::kBoruvkaSpan;
+  Block k;
+  k.take(&b.cnt, V);
+  k.take(&b.fill, V);
+  k.take(&b.packed, V);
+  k.take(&b.scan_total, 1);
+  k.take(&b.scan_tmp, gz::scan_tmp_words(V));
+  k.take(&b.order, V);
+  k.take(&b.order_comp, V);
+  k.take(&b.comp_start, V + 1);
+  k.take(&b.comp_key, V);
+  k.take(&b.ncomp, 1);
+  k.take(&b.acc, (warps + 1) * acc_words);
+  k.take(&b.part, warps * acc_words);
+  k.take(&b.part_comp, warps);
+  k.take(&b.big, 1);
+  k.take(&b.cross, warps + 1);
+  k.take(&b.ncross, 1);
+  return k.alloc(&b.block_phases);
+}
+
 void free_bv(gz::BoruvkaBufs &b) {
-  dev_free(b.parent);
-  dev_free(b.label);
-  dev_free(b.cnt);
-  dev_free(b.fill);
-  dev_free(b.minv);
-  dev_free(b.packed);
-  dev_free(b.scan_total);
-  dev_free(b.scan_tmp);
-  dev_free(b.order);
-  dev_free(b.order_comp);
-  dev_free(b.comp_start);
-  dev_free(b.comp_key);
-  dev_free(b.ncomp);
-  dev_free(b.acc);
-  dev_free(b.part);
-  dev_free(b.part_comp);
-  dev_free(b.big);
-  dev_free(b.round);
-  b.ctl = nullptr;
-  dev_free(b.flags);
-  dev_free(b.cross);
-  dev_free(b.ncross);
-  dev_free(b.qbar);
-  dev_free(b.btot);
-  dev_free(b.forest);
-  dev_free(b.forest_n);
-  dev_free(b.trace_n);
+  dev_free(b.block);
+  dev_free(b.block_phases);
+  dev_free(b.block_query);
+  if (b.trace) cudaFree(b.trace);
+  b = gz::BoruvkaBufs{};
 }
 
 // boruvka_emulation (src/cc_sketch_alg.cpp:464-513) on the sketches at sk with buffers b: the
 // query graph (every round on the device, no host round trip) enqueued on stream s, then the
 // rounds, the out-of-samples flag and the component count copied to pin[0..2] (pinned).
-// The query mode in effect. By size: the one-launch query up to 2^18 vertices (a round's phases
-// are short there, and launches and gaps between them dominated: 0.59 against 0.64 ms at 2^17);
-// the graph of per-phase kernels above (each phase then has work for more resident warps than the
-// cooperative kernel's registers allow: 1.8-2.0 against 2.1-2.2 ms per query at 2^20).
-constexpr uint32_t kOneLaunchQueryMaxV = 1u << 18;
+// The query mode in effect. By size: the one-launch query up to 2^21 vertices (a blocking query over
+// the first tenth of a power-law stream at 2^20 vertices: 1.43 ms against 2.02 ms for the graph of
+// per-phase kernels; at 2^16: 0.18 against 0.47). Its per-root accumulators take 3.5% of the
+// sketches' size; past 2^21 vertices (1 GB of them), or where they cannot be allocated, the graph.
+constexpr uint32_t kOneLaunchQueryMaxV = 1u << 21;
 int query_mode_of(const gz_alg *h) {
-  if (h->query_mode >= 0) return h->query_mode;
-  return h->V <= kOneLaunchQueryMaxV ? 2 : 1;
+  const int mode = h->query_mode >= 0 ? h->query_mode : h->V <= kOneLaunchQueryMaxV ? 2 : 1;
+  return mode == 2 && h->no_one_launch ? 1 : mode;
+}
+
+// Buffers of the query mode in effect; when those of the one-launch query cannot be had, the
+// handle's queries run as the graph.
+int bv_ensure_mode(gz_alg *h, gz::BoruvkaBufs &b, cudaStream_t s) {
+  if (query_mode_of(h) == 2 && !b.block_query) {
+    Block k;
+    k.take(&b.racc, gz::query_racc_words(h->V, h->cps, h->B));
+    k.take(&b.rstate, 2 * (size_t)h->V);
+    k.take(&b.det, 4 * (size_t)h->V);
+    k.take(&b.qbar, 1);
+    k.take(&b.racc_dirty, 1);
+    if (k.alloc(&b.block_query) == GZ_OK) {
+      GZ_CUDA(cudaMemsetAsync(b.racc_dirty, 0xff, sizeof(uint32_t), s));
+    } else {
+      cudaGetLastError();  // the failed allocation must not surface in a later launch's check
+      h->no_one_launch = true;
+    }
+  }
+  if (query_mode_of(h) != 2) return alloc_bv_phases(b, h->V, (size_t)(h->cps * h->B + 1) * 3);
+  return GZ_OK;
 }
 
 int boruvka_enqueue(gz_alg *h, gz::BoruvkaGraph &q, const gz::BoruvkaGeom &g, const uint8_t *sk,
                     gz::BoruvkaBufs &b, uint32_t *d_final, uint32_t *d_ncc, uint32_t *pin,
                     cudaStream_t s) {
+  GZ_TRY(bv_ensure_mode(h, b, s));
   const int mode = query_mode_of(h);
-  if (mode == 2) GZ_CUDA(gz::boruvka_query_launch(g, h->samples, sk, b, d_final, d_ncc, s));
+  if (mode == 2) GZ_CUDA(gz::boruvka_query_launch(g, h->samples, sk, b, 0, d_final, d_ncc, s));
   else if (mode == 1) GZ_CUDA(gz::boruvka_graph_launch(q, g, h->samples, sk, b, d_final, d_ncc, s));
   else GZ_CUDA(gz::boruvka_host_loop(g, h->samples, sk, b, d_final, d_ncc, pin, s));
   GZ_CUDA(cudaMemcpyAsync(pin, b.ctl, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -949,10 +954,7 @@ std::string out_of_samples_msg(const gz_alg *h, uint32_t round) {
 int tickets_ensure(gz_alg *h) {
   auto &T = h->tq;
   if (T.d_final) return GZ_OK;
-  GZ_TRY(alloc_bv(T.bv, h->V, (size_t)(h->cps * h->B + 1) * 3, h->d_status));
-  GZ_TRY(dev_alloc(&T.d_ncc, 1));
-  GZ_TRY(dev_alloc(&T.d_final, h->V));
-  return GZ_OK;
+  return alloc_bv(T.bv, h->V, h->d_status, &T.d_final, &T.d_ncc);
 }
 
 void ticket_free(gz_alg::Ticket &t) {
@@ -971,16 +973,13 @@ void tickets_shutdown(gz_alg *h) {
   T.pool.clear();
   gz::boruvka_graph_free(T.graph);
   free_bv(T.bv);
-  dev_free(T.d_final);
-  dev_free(T.d_ncc);
+  T.d_final = T.d_ncc = nullptr;
 }
 
 int ensure_query(gz_alg *h) {
   auto &b = h->bv;
   const size_t V = h->V;
-  GZ_TRY(alloc_bv(b, V, (size_t)(h->cps * h->B + 1) * 3, h->d_status));
-  GZ_TRY(dev_alloc(&h->d_final, V));
-  GZ_TRY(dev_alloc(&h->d_ncc, 1));
+  GZ_TRY(alloc_bv(b, V, h->d_status, &h->d_final, &h->d_ncc));
   if (h->trace && !b.trace) {
     const size_t cap = V * (size_t)(h->C + 1);
     void *p = nullptr;
@@ -1426,8 +1425,8 @@ int gz_query_submit(gz_alg_t *h, uint64_t *ticket) {
     }
   }
   const int pi = h->prof_begin();
-  t.graph = query_mode_of(h) == 1;
   int rc = boruvka_enqueue(h, T.graph, h->bgeom(), h->d_sk, T.bv, T.d_final, T.d_ncc, t.pin, h->stream);
+  t.graph = query_mode_of(h) == 1;
   h->prof_end(pi, 2);
   cudaError_t e = cudaSuccess;
   if (rc == GZ_OK) e = cudaMemcpyAsync(t.labels, T.d_final, sizeof(uint32_t) * h->V, cudaMemcpyDeviceToHost, h->stream);
@@ -1534,11 +1533,12 @@ int gz_spanning_forest(gz_alg_t *h, uint32_t *edges_out, size_t cap, size_t *n_e
   GZ_CUDA(cudaMemcpyAsync(h->h_status + 3, h->bv.forest_n, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
   GZ_CUDA(cudaStreamSynchronize(h->stream));
   n = std::min<uint32_t>(h->h_status[3], h->V);
-  *n_edges = n;
-  if (edges_out && cap) {
-    std::vector<uint64_t> idx(n);
-    if (n) GZ_CUDA(cudaMemcpy(idx.data(), h->bv.forest, n * sizeof(uint64_t), cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < std::min<size_t>(cap, n); ++i) {
+  std::vector<uint64_t> idx(n);
+  if (n) GZ_CUDA(cudaMemcpy(idx.data(), h->bv.forest, n * sizeof(uint64_t), cudaMemcpyDeviceToHost));
+  idx.erase(std::remove(idx.begin(), idx.end(), gz::kNoEdge), idx.end());
+  *n_edges = idx.size();
+  if (edges_out) {
+    for (size_t i = 0; i < std::min(cap, idx.size()); ++i) {
       edges_out[2 * i] = (uint32_t)(idx[i] >> 32);
       edges_out[2 * i + 1] = (uint32_t)idx[i];
     }

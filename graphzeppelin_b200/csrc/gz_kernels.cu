@@ -703,11 +703,9 @@ __global__ void k_bv_reset(uint32_t V, uint32_t *parent) {
   if (v < V) parent[v] = v;
 }
 
-// The Boruvka phases below are device functions shared by the per-phase kernels (one launch
-// each, the CUDA-graph and host-loop queries) and by k_bv_query (every phase of every round in
-// one cooperative launch). Data written earlier in the same query is read through L2 (__ldcg):
-// in k_bv_query another SM wrote it in an earlier phase of the same kernel. A warp's copy ring
-// counts its batches in T across calls, so its two mbarriers' phases stay in step.
+// The Boruvka phases below are the per-phase kernels of the CUDA-graph and host-loop queries (the
+// one-launch query is gz_query.cu). A warp's copy ring counts its batches in T across calls, so
+// its two mbarriers' phases stay in step.
 
 // Round 0 (run_round_zero, src/cc_sketch_alg.cpp:223-244) for warp gw of nwarps: every vertex
 // sketch samples its sample 0 -- columns 0..CPS-1 and the deterministic bucket. The warp takes
@@ -1301,207 +1299,6 @@ __global__ void k_bv_final(uint32_t V, uint32_t *parent, uint32_t *out, uint32_t
   if (v < V) bv_final_vertex(v, parent, out, ncc);
 }
 
-// ---- the whole query in one cooperative launch ------------------------------------------------
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Grid-wide barrier of a cooperative launch: the blocks count their arrivals in *count (zeroed
-// before the launch); barrier number k completes at k * gridDim.x arrivals. Writes before it are
-// seen by every block after it (fence, arrival, acquire, fence). A block with a failed warp
-// (failed = true in any thread) leaves without arriving; a block that waits longer than
-// kWaitLimitNs sets the timeout status. Both return false, and the caller returns from the kernel
-// (the other blocks then time out at their next barrier).
-__device__ bool grid_barrier(uint32_t *count, uint32_t k, bool failed, uint32_t *status) {
-  __shared__ uint32_t s_ok;
-  if (__syncthreads_or(failed)) return false;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(count, 1u);
-    const uint32_t target = k * gridDim.x;
-    uint32_t ok = 1;
-    if (ld_acquire_gpu(count) < target) {
-      const uint64_t t0 = global_ns();
-      while (ld_acquire_gpu(count) < target) {
-        if (global_ns() - t0 > kWaitLimitNs) {
-          atomicOr(status, kStatusTimeout);
-          ok = 0;
-          break;
-        }
-        __nanosleep(32);
-      }
-    }
-    __threadfence();
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// Batches of the one-launch query's copy rings: NS - 1 of them in flight while one is read (a
-// third batch measured no faster than two).
-constexpr int kBvQueryRing = 2;
-
-// Exclusive scan of one u64 per thread over a block of 256 threads.
-__device__ __forceinline__ uint64_t block_scan_u64_256(uint64_t x, uint64_t *ws /*8*/) {
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint64_t inc = x;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint64_t y = __shfl_up_sync(kFull, inc, o);
-    if (lane >= (uint32_t)o) inc += y;
-  }
-  if (lane == 31) ws[warp] = inc;
-  __syncthreads();
-  uint64_t pre = 0;
-  for (uint32_t k = 0; k < warp; ++k) pre += ws[k];
-  __syncthreads();
-  return pre + inc - x;
-}
-
-// boruvka_emulation (src/cc_sketch_alg.cpp:464-513) in one cooperative launch of 256-thread
-// blocks: a fresh DSU, round 0, then per round the phases of the per-phase kernels separated by
-// grid barriers -- (1) roots and members per root; (2) each block's exclusive scan of (members |
-// 1 << 32) over its range of CH vertices; (3) each block's scan of the blocks' totals, then the
-// grouping; (4) the merge over spans, sampling the components inside a span, with the next round's
-// counters cleared; (5) the partial slots folded; (6) the components crossing span edges sampled
-// -- then the loop test of k_bv_check, taken by every block alike, and the labels. A round's
-// "modified" word is b.flags[round % 3]: the word of round r + 1 is cleared during round r, long
-// after every block read it as the word of round r - 2.
-template <int CPS, int NW, int KB, int KBP>
-__global__ void __launch_bounds__(256) k_bv_query(BoruvkaGeom g, const uint32_t *__restrict__ sk_words,
-                                                  BoruvkaBufs b, uint32_t samples,
-                                                  uint32_t *labels_out, uint32_t *ncc) {
-  extern __shared__ __align__(16) uint8_t bv_smem[];
-  __shared__ uint64_t s_pref[kBvQueryMaxBlocks + 1];
-  __shared__ uint64_t s_ws[8];
-  __shared__ RootTable tab;
-  const uint32_t V = g.V, nblk = gridDim.x, tid = threadIdx.x;
-  const uint32_t W = 3 * CPS * g.B;
-  BvRingN<kBvQueryRing> ring;
-  ring.init(bv_smem + (tid >> 5) * bv_warp_bytes(W, KB, kBvQueryRing), W, KB);
-  uint32_t T = 0;     // batches through this warp's copy ring
-  uint32_t nbar = 0;  // grid barriers passed
-  bool failed = false;
-  auto sync = [&]() { return grid_barrier(b.qbar, ++nbar, failed, b.status); };
-  const uint32_t gw = (blockIdx.x * blockDim.x + tid) >> 5, nwarps = (nblk * blockDim.x) >> 5;
-  const uint32_t gt = blockIdx.x * blockDim.x + tid, nthreads = nblk * blockDim.x;
-  uint32_t *minv = b.trace ? b.minv : nullptr;
-  for (uint32_t v = gt; v < V; v += nthreads) {
-    b.parent[v] = v;
-    b.cnt[v] = 0;
-    b.fill[v] = 0;
-    if (minv) minv[v] = 0xffffffffu;
-  }
-  if (gt == 0) {
-    *b.forest_n = 0;
-    if (b.trace) *b.trace_n = 0;
-    b.flags[0] = b.flags[1] = b.flags[2] = 0;
-    *b.big = 0xffffffffu;
-    *b.ncross = 0;
-    *ncc = 0;
-  }
-  if (!sync()) return;
-  failed = !bv_round0_warp<CPS, KB, kBvQueryRing>(g, sk_words, b, b.flags, ring, T, gw, nwarps);
-  if (!sync()) return;
-  const uint32_t CH = (((V + nblk - 1) / nblk) + 255) & ~255u;  // scan range of a block
-  const uint32_t nspans = (V + g.span - 1) / g.span;
-  const uint32_t acc_words = (CPS * g.B + 1) * 3;
-  uint32_t round = 0;
-  for (;;) {
-    const uint32_t modified = __ldcg(b.flags + round % 3);
-    if (modified == 0 || round + 1 >= samples) {
-      if (gt == 0) {
-        b.ctl[0] = modified ? round + 1 : round;
-        b.ctl[1] = modified ? 1u : 0u;
-        b.ctl[2] = 0;
-        *b.round = round;
-      }
-      break;
-    }
-    ++round;
-    uint32_t *flags = b.flags + round % 3;
-    // (1)
-    if (gt == 0) {
-      b.flags[(round + 1) % 3] = 0;
-      if (round > 1) *b.ncross = 0;  // the previous round's list was read before the last barrier
-    }
-    for (uint32_t v0 = blockIdx.x * 512; v0 < V; v0 += nblk * 512)
-      bv_label_block<2>(V, v0, b.parent, b.label, b.cnt, minv, tab);
-    if (!sync()) return;
-    // (2)
-    {
-      const uint32_t ipt = CH / 256, a = blockIdx.x * CH + tid * ipt;
-      uint64_t sum = 0;
-      for (uint32_t i = 0; i < ipt; ++i)
-        if (a + i < V) {
-          const uint32_t c = __ldcg(b.cnt + a + i);
-          sum += (uint64_t)c | (c ? (1ull << 32) : 0ull);
-        }
-      uint64_t run = block_scan_u64_256(sum, s_ws);
-      for (uint32_t i = 0; i < ipt; ++i)
-        if (a + i < V) {
-          const uint32_t c = __ldcg(b.cnt + a + i);
-          b.packed[a + i] = run;
-          run += (uint64_t)c | (c ? (1ull << 32) : 0ull);
-        }
-      if (tid == 255) b.btot[blockIdx.x] = run;
-    }
-    if (!sync()) return;
-    // (3)
-    {
-      const uint32_t per = (nblk + 255) / 256;
-      uint64_t sum = 0;
-      for (uint32_t k = 0; k < per; ++k) {
-        const uint32_t i = tid * per + k;
-        if (i < nblk) sum += __ldcg(b.btot + i);
-      }
-      uint64_t run = block_scan_u64_256(sum, s_ws);
-      for (uint32_t k = 0; k < per; ++k) {
-        const uint32_t i = tid * per + k;
-        if (i < nblk) {
-          s_pref[i] = run;
-          run += __ldcg(b.btot + i);
-        }
-      }
-      if (tid == 255) s_pref[nblk] = run;
-      __syncthreads();
-      const uint32_t nc = (uint32_t)(s_pref[nblk] >> 32);
-      for (uint32_t v0 = blockIdx.x * 512; v0 < V; v0 += nblk * 512)
-        bv_group_block<2>(V, v0, acc_words, g.span, b.label,
-                       [&](uint32_t r) { return __ldcg(b.packed + r) + s_pref[r / CH]; }, nc, b.cnt,
-                       b.fill, minv, b.order, b.order_comp, b.comp_start, b.comp_key, b.ncomp,
-                       b.acc, b.big, b.cross, b.ncross, tab);
-    }
-    if (!sync()) return;
-    // (4)
-    for (uint32_t w = gw; w < nspans && !failed; w += nwarps)
-      failed = !bv_merge_span<CPS, NW, KB, kBvQueryRing>(g, sk_words, b, round, flags, ring, T, w);
-    for (uint32_t v = gt; v < V; v += nthreads) {
-      b.cnt[v] = 0;
-      b.fill[v] = 0;
-      if (minv) minv[v] = 0xffffffffu;
-    }
-    if (!sync()) return;
-    // (5)
-    for (uint32_t s0 = gw * kPartsPerWarp; s0 < nspans; s0 += nwarps * kPartsPerWarp)
-      bv_reduce_parts_warp<CPS, NW, KBP>(g, nspans, b, s0, kPartsPerWarp);
-    if (gt == 0) *b.big = 0xffffffffu;
-    if (!sync()) return;
-    // (6)
-    const uint32_t nx = __ldcg(b.ncross);
-    for (uint32_t i = gw; i < nx; i += nwarps)
-      bv_sample_spanning_comp<CPS>(g, b, round, flags, __ldcg(b.cross + i));
-    if (!sync()) return;
-  }
-  for (uint32_t v = gt; v < V; v += nthreads) bv_final_vertex(v, b.parent, labels_out, ncc);
-}
-
-// Shared-memory bucket-update probe: every thread XORs 96-bit updates into random 12-byte
-// buckets of a 16-vertex staged tile with three 32-bit atomicXor each -- the sketch-update
-// kernel's per-bucket operation, without hashing or global traffic.
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -1832,41 +1629,6 @@ cudaError_t boruvka_round(const BoruvkaGeom &g, const uint8_t *sketches, const B
   else k_bv_sample_spanning<7><<<sblocks, 256, 0, s>>>(g, b);
   g_launches++;
   return cudaGetLastError();
-}
-
-constexpr int kBvQueryBlocksPerSm = 4;
-
-cudaError_t boruvka_query_launch(const BoruvkaGeom &g, uint32_t samples, const uint8_t *sketches,
-                                 const BoruvkaBufs &b, uint32_t *labels_out, uint32_t *ncc,
-                                 cudaStream_t s) {
-  const size_t smem = 8 * (size_t)bv_warp_bytes(3 * g.cps * g.B, bv_batch(g.cps), kBvQueryRing);
-  auto launch = [&](auto kern) -> cudaError_t {
-    cudaError_t e = smem_optin(kern);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    // every block resident at once (the launch fails otherwise): a grid barrier never waits for
-    // a block that has not started
-    const int blocks = std::min<int>(std::min(per_sm, kBvQueryBlocksPerSm) * num_sms(), (int)kBvQueryMaxBlocks);
-    e = cudaMemsetAsync(b.qbar, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    BoruvkaGeom a_g = g;
-    const uint32_t *a_sk = reinterpret_cast<const uint32_t *>(sketches);
-    BoruvkaBufs a_b = b;
-    uint32_t a_samples = samples;
-    uint32_t *a_labels = labels_out, *a_ncc = ncc;
-    void *args[] = {&a_g, &a_sk, &a_b, &a_samples, &a_labels, &a_ncc};
-    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(blocks), dim3(256), args,
-                                    smem, s);
-    g_launches++;
-    return e;
-  };
-  if (g.cps == 1 && g.B <= 42) return launch(k_bv_query<1, 4, 8, 4>);
-  if (g.cps == 1) return launch(k_bv_query<1, 6, 8, 4>);
-  if (g.cps == 7) return launch(k_bv_query<7, dev::Region<7>::kNW, 1, 1>);
-  return cudaErrorInvalidValue;
 }
 
 cudaError_t boruvka_final(const BoruvkaGeom &g, const BoruvkaBufs &b, uint32_t *labels_out,

@@ -191,7 +191,10 @@ cudaError_t sketch_xor_raw(uint8_t *sketches, uint32_t sketch_words, uint32_t v,
                            const uint32_t *raw, cudaStream_t s);
 
 // ---- Boruvka -----------------------------------------------------------------------------------
+constexpr uint64_t kNoEdge = ~0ull;  // never an edge index (vertex ids are below 2^31)
 struct BoruvkaBufs {
+  // the allocations that the arrays below are cut from
+  uint8_t *block = nullptr, *block_phases = nullptr, *block_query = nullptr;
   uint32_t *parent;      // V   DSU parents
   uint32_t *label;       // V   root per vertex for the current round
   uint32_t *cnt;         // V   members per root
@@ -212,26 +215,27 @@ struct BoruvkaBufs {
   uint32_t *big;         // 1   the component holding more than half the vertices, or ~0
   uint32_t *round;       // 1   the current round (device-driven loop)
   uint32_t *ctl;         // 3   after the loop: rounds run, out of samples (0/1); go on (0/1)
-  uint32_t *flags;       // [0] modified (k_bv_query: [round % 3])
+  uint32_t *flags;       // [0] modified (one-launch query: [round % 3])
   uint32_t *cross;       // V / span + 1  components crossing a span edge (sampled from acc)
   uint32_t *ncross;      // 1
-  uint32_t *qbar;        // 1   arrivals at the grid barriers of k_bv_query
-  uint64_t *btot;        // kBvQueryMaxBlocks  per-block totals of k_bv_query's scan
-  uint64_t *forest;      // V   spanning-forest edge indices
-  uint32_t *forest_n;    // 1
+  // one-launch query (null in the buffers of the per-phase kernels)
+  uint32_t *qbar;        // 1   arrivals at its grid barriers
+  uint32_t *rstate;      // 2V  per root: 1 + last round it sampled ZERO / was linked to
+  uint32_t *racc;        // V x query_racc_words: per root, its component's merged sample
+  uint32_t *det;         // 4V  deterministic buckets, 16 bytes each
+  uint32_t *racc_dirty;  // 1   racc may hold leftovers (first use; a query that did not finish)
+  uint64_t *forest;      // V   spanning-forest edge indices (entries of kNoEdge are empty)
+  uint32_t *forest_n;    // 1   entries in use, empty ones included
   void *trace;           // gz_trace_rec_t[trace_cap] or null
   uint32_t *trace_n;     // 1
   uint32_t trace_cap;
+  uint32_t pad;          // compared bytewise with the rest (boruvka_graph_launch)
   uint32_t *status;
 };
 
 // Bytes allocated past the last vertex sketch of any sketch buffer a query reads: its bulk copies
 // read 16-byte-aligned supersets of bucket runs, up to 15 bytes beyond the last sketch.
 constexpr size_t kSketchTail = 256;
-
-// Blocks of the one-launch query (k_bv_query), at most: per-block scan totals are kept for
-// each, and each block scans all of them in shared memory.
-constexpr uint32_t kBvQueryMaxBlocks = 1184;
 
 // Grouped members XOR-merged by one warp per Boruvka round (the per-warp partial slots are
 // sized by it).
@@ -246,6 +250,7 @@ struct BoruvkaGeom {
   // sketches is zero and a component's merged sketch equals the XOR over all other vertices:
   // the largest component (over half the vertices) is merged from its complement.
   uint32_t complement = 0;
+  uint32_t pad = 0;  // compared bytewise with the rest (boruvka_graph_launch)
 };
 
 // XOR of every vertex sketch, word by word, into total[sketch_words] (zeroed by the caller).
@@ -284,15 +289,18 @@ void boruvka_graph_free(BoruvkaGraph &q);
 // The same kernels with the loop run from the host (a device-to-host copy and a synchronize per
 // round; for profilers that do not see kernels inside conditional graphs). Leaves b.ctl[0..1]
 // as the graph does; pin is pinned host memory of at least 3 words.
-// boruvka_emulation in one cooperative kernel launch (all rounds on the device, grid barriers
-// between the phases of a round): the same answer, rounds, samples and trace as the graph and the
-// host loop. b.ctl then holds the rounds and the out-of-samples flag.
-cudaError_t boruvka_query_launch(const BoruvkaGeom &g, uint32_t samples, const uint8_t *sketches,
-                                 const BoruvkaBufs &b, uint32_t *labels_out, uint32_t *ncc,
-                                 cudaStream_t s);
 cudaError_t boruvka_host_loop(const BoruvkaGeom &g, uint32_t samples, const uint8_t *sketches,
                               const BoruvkaBufs &b, uint32_t *labels_out, uint32_t *ncc,
                               uint32_t *pin, cudaStream_t s);
+
+// boruvka_emulation in one kernel launch (gz_query.cu; all rounds on the device, barriers over the
+// launch between the phases of a round): the same answer, rounds, samples and trace as the graph
+// and the host loop. b.ctl then holds the rounds and the out-of-samples flag. When *b.status has
+// a bit of abort_mask set as the kernel starts, the query is not run and nothing is written.
+cudaError_t boruvka_query_launch(const BoruvkaGeom &g, uint32_t samples, const uint8_t *sketches,
+                                 const BoruvkaBufs &b, uint32_t abort_mask, uint32_t *labels_out,
+                                 uint32_t *ncc, cudaStream_t s);
+size_t query_racc_words(uint32_t V, uint32_t cps, uint32_t B);  // words of BoruvkaBufs::racc
 
 int num_sms();
 // columns C and buckets per column B of one vertex sketch for V vertices and sketches factor f

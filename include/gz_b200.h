@@ -307,12 +307,14 @@ GZ_API int gz_set_tuning(gz_alg_t *alg, uint32_t vertices_per_tile, uint32_t thr
  * staging it in shared memory against updating its buckets in HBM -- is updated in place with
  * global atomics. 0 = always staged, 1 = the default. Same role as gz_batch_set_route. */
 GZ_API int gz_set_direct_factor(gz_alg_t *alg, double factor);
-/* How queries run. mode = 2: the whole Boruvka emulation in one cooperative kernel launch, every
- * round on the device with grid barriers between its phases. mode = 1: one CUDA graph of
- * per-phase kernels whose conditional while node loops over the rounds. mode = 0: the same
- * per-phase kernels with the round loop on the host (a synchronize per round; ticket submits then
- * wait for their query), for profilers that do not see kernels inside conditional graphs.
- * mode = -1 (the default): 2 up to 2^18 vertices, 1 above (the faster of the two at each size).
+/* How queries run. mode = 2: the whole Boruvka emulation in one kernel launch, every round on the
+ * device with barriers over the launch between its phases (one thread-block cluster for small
+ * graphs, else a cooperative launch). mode = 1: one CUDA graph of per-phase kernels whose
+ * conditional while node loops over the rounds. mode = 0: the same per-phase kernels with the
+ * round loop on the host (a synchronize per round; ticket submits then wait for their query), for
+ * profilers that do not see kernels inside conditional graphs. mode = -1 (the default): 2 up to
+ * 2^21 vertices, 1 above. Mode 2 keeps one sample per vertex as workspace (3.5% of the sketches);
+ * where that cannot be allocated the handle's queries run as mode 1.
  * Answers, rounds and sample traces are the same in every mode. GZ_ERR_INVALID for another mode. */
 GZ_API int gz_set_query_graph(gz_alg_t *alg, int mode);
 /* Sketch-update kernel of a handle: mode 1 = the tile pipeline (a producer warp loads the next
