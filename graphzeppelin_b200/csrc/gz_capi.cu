@@ -153,6 +153,9 @@ struct gz_alg {
   int planes_mode = -1;         // entry form asked for: -1 automatic, 0 plain, 1 coded (4-bit
                                 // codes where they fit, else 3-bit), 2 coded with 3-bit codes
   gz::PlaneHash ph{};
+  // plain entries applied through bucket planes, hashed there (handles without coded entries)
+  bool plain_planes = false;
+  gz::PlaneHashWide phw{};
   gz::ChunkTable chunks{};
   int nchunks = 0;
   uint32_t *d_bin_off = nullptr;
@@ -239,7 +242,7 @@ struct gz_alg {
     // Staging a tile moves its sketches twice (bulk load + write-back); updating it in place
     // costs about C + 1 bucket sectors read and written per entry. Below the break-even entry
     // count a tile goes in place (one tile per bin and plain CameoSketch entries only).
-    if (bin_shift == tile_shift && !cube && !planes) {
+    if (bin_shift == tile_shift && !cube && !planes && !plain_planes) {
       const double even = (double)((uint64_t)nb * 12 << tile_shift) / (32.0 * (C + 1));
       g.direct_max = (uint32_t)std::min(even * direct_factor, 4.0e9);
     }
@@ -248,6 +251,7 @@ struct gz_alg {
   gz::GutterGeom ggeom() const { return gz::GutterGeom{V, bin_shift, nbins}; }
   gz::PlaneGeom pgeom() const {
     gz::PlaneGeom g;
+    g.groups = (C + gz::kPlaneSlots) / gz::kPlaneSlots;
     g.V = V;
     g.C = C;
     g.B = B;
@@ -262,8 +266,14 @@ struct gz_alg {
     const double wb = 24.0 * ((double)C * std::min<uint32_t>(B, gz::kPlaneRows - 1) + 1) *
                       (double)(1u << tile_shift);
     const double even = wb / (64.0 * (C + 1));
-    g.direct_max = (uint32_t)std::min(even * direct_factor, 4.0e9);
+    g.direct_max = cube || g.groups > 1 ? 0 : (uint32_t)std::min(even * direct_factor, 4.0e9);
     return g;
+  }
+  // Records of one call that go straight to the sketches: when the call brings so few that most of
+  // its tiles would be updated in place anyway, one launch without a gutter does it.
+  bool direct_call(uint64_t n) const {
+    if (cube || C > gz::kPlaneMaxColumns || !(planes || plain_planes)) return false;
+    return 2.0 * (double)n < (double)pgeom().direct_max * ntiles;
   }
   gz::BoruvkaGeom bgeom() const {
     gz::BoruvkaGeom g;
@@ -368,7 +378,10 @@ int choose_planes(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tp
   // By default past 2^18 vertices the pipelined staged kernel stays in use (large sparse graphs,
   // where a wave brings few entries per tile)
   if (!asked && h->V > kPlaneDefaultMaxV) return GZ_OK;
-  const uint32_t shift = vpt_req ? (uint32_t)__builtin_ctz(vpt_req) : 5;
+  // Tiles of 32 vertices, fewer where that leaves SMs without a tile or two (a call is then as long as
+  // its last wave: 1,024 vertices, 8,528 records: 18 us in tiles of 32, 9 us in tiles of 8)
+  uint32_t shift = vpt_req ? (uint32_t)__builtin_ctz(vpt_req) : 5;
+  while (!vpt_req && !tpb_req && !threads_req && shift > 3 && (h->V >> shift) < 2u * gz::num_sms()) --shift;
   uint32_t bshift = shift;
   if (tpb_req) {
     bshift = shift + (uint32_t)__builtin_ctz(tpb_req);
@@ -390,7 +403,7 @@ int choose_planes(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tp
     if (asked) return fail(GZ_ERR_INVALID, "the codes of this sketch do not fit a 16-byte coded entry");
     return GZ_OK;
   }
-  uint32_t threads = threads_req ? threads_req : 1024;
+  uint32_t threads = threads_req ? threads_req : vpt_req ? 1024 : (uint32_t)gz::plane_threads(shift);
   if (threads_req && (threads_req < 64 || threads_req > 1024 || threads_req % 32))
     return fail(GZ_ERR_INVALID, "threads_per_block must be a multiple of 32 in [64, 1024]");
   if (gz::plane_update_smem(shift, (int)threads) > h->smem_optin)
@@ -415,6 +428,7 @@ int choose_tiling(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tp
   if (smem_optin <= 0) smem_optin = 227 * 1024;
   h->smem_optin = (size_t)smem_optin;
   h->planes = false;
+  h->plain_planes = false;
   h->codes3 = false;
   h->threads = 1024;
   {
@@ -446,6 +460,21 @@ int choose_tiling(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tp
   }
   // two-buffer pipeline: two tiles (one bin each) and the hash constants in shared memory
   h->pipe = false;
+  // Left to itself, a handle without coded entries applies its plain entries through bucket planes:
+  // tiles of 8 vertices (four CTAs an SM) with a gutter bin each, of 16 or 32 where that many more
+  // vertices still keep the bins within the shared-memory sort. Against staging whole tiles: 2^20
+  // vertices, 1.28e7 records 5.5 -> 4.5 ms; CubeSketch, 5,003 vertices, 1e6 records 3.7 -> 0.54 ms.
+  if (!h->in_place && h->planes_mode < 0 && h->pipe_mode < 0 && !vpt_req && !threads_req && !tpb_req &&
+      h->C <= gz::kPlaneMaxColumnsWide) {
+    shift = 3;
+    while (shift < 5 && (h->V >> shift) >= gz::kSortBinsMax && (h->V >> 5) < gz::kSortBinsMax) ++shift;
+    h->plain_planes = true;
+    h->phw = gz::plane_hash_wide(h->seed, h->C, h->B);
+    h->tile_shift = h->bin_shift = shift;
+    h->ntiles = h->nbins = (uint32_t)((h->V + (1u << shift) - 1) >> shift);
+    h->threads = (uint32_t)gz::plane_threads(shift);
+    return GZ_OK;
+  }
   if (!h->in_place && !h->cube && !tpb_req && want_pipe(h)) {
     const size_t room = (size_t)smem_optin - 1024 - (((size_t)h->C + 2) & ~(size_t)1) * 8;
     // the most buffers asked for (or kPipeBuffers) that hold tiles of at least 4 vertices
@@ -614,6 +643,9 @@ int apply_pending(gz_alg *h) {
     const int grid = (int)std::min<uint64_t>(h->ntiles, (uint64_t)gz::num_sms() * per_sm);
     GZ_CUDA(gz::plane_update(h->pgeom(), h->ph, h->d_sk, h->d_gutter, h->chunks, h->d_bin_off,
                              h->nchunks, h->d_status + 1, h->d_status, grid, (int)h->threads, h->stream));
+  } else if (h->plain_planes) {
+    GZ_CUDA(gz::plane_update_plain(h->pgeom(), h->cube, h->phw, h->d_sk, h->d_gutter, h->chunks, h->d_bin_off,
+                                   h->nchunks, h->d_status + 1, h->stream));
   } else if (h->pipe) {
     const int grid = (int)std::min<uint64_t>(h->ntiles, (uint64_t)gz::num_sms());
     GZ_CUDA(gz::sketch_update_pipe(g, h->d_sk, h->d_gutter, h->chunks, h->d_bin_off, h->nchunks, h->d_flip,
@@ -639,6 +671,13 @@ int gutter_chunk(gz_alg *h, int input, const void *d_in, uint64_t n) {
     const int pi = h->prof_begin();
     GZ_CUDA(gz::apply_in_place(input, d_in, n, h->sgeom(), h->d_sk, h->d_flip, h->d_status, h->stream));
     h->prof_end(pi, 1);
+    return GZ_OK;
+  }
+  if (input == gz::kInputRecords && h->direct_call(n)) {
+    const int pi = h->prof_begin();
+    GZ_CUDA(gz::direct_records(d_in, n, h->V, h->nb * 3, h->ph, h->d_sk, h->d_status, h->stream));
+    h->prof_end(pi, 1);
+    h->prof_acc.entries_applied += 2 * n;
     return GZ_OK;
   }
   const uint64_t per = input == gz::kInputRecords ? 2 : 1;
@@ -671,7 +710,7 @@ int gutter_chunk(gz_alg *h, int input, const void *d_in, uint64_t n) {
   GZ_CUDA(gz::gutter_bin_offsets(h->d_hist, 1, h->nbins, h->d_total, bin_off, h->stream));
   if (coded) {
     // records -> coded entries, each record hashed once
-    const uint32_t tile = gz::hash_sort_tile(h->nbins, h->smem_optin - 1024);
+    const uint32_t tile = gz::hash_sort_tile(h->nbins, h->smem_optin - 1024, n);
     if (tile == 0) return fail(GZ_ERR_INVALID, "gutter bins do not fit the hash sort");
     GZ_CUDA(cudaMemsetAsync(h->d_fill, 0, sizeof(uint32_t) * h->nbins, h->stream));
     GZ_CUDA(gz::gutter_hash_sort(d_in, n, gg, h->ph, tile, h->d_hist, h->d_fill,
@@ -1731,7 +1770,7 @@ int gz_set_tuning(gz_alg_t *h, uint32_t vpt, uint32_t threads, uint32_t tiles_pe
   GZ_TRY(apply_pending(h));
   GZ_CUDA(cudaStreamSynchronize(h->stream));
   const int keep_mode = h->planes_mode;
-  const bool keep_planes = h->planes, keep_pipe = h->pipe, keep_codes3 = h->codes3;
+  const bool keep_planes = h->planes, keep_pipe = h->pipe, keep_codes3 = h->codes3, keep_plain = h->plain_planes;
   const uint32_t keep[5] = {h->tile_shift, h->ntiles, h->bin_shift, h->nbins, h->threads};
   h->planes_mode = entry_form == 0 ? -1 : (int)entry_form - 1;
   const uint32_t old_nb = h->nbins;
@@ -1739,6 +1778,7 @@ int gz_set_tuning(gz_alg_t *h, uint32_t vpt, uint32_t threads, uint32_t tiles_pe
   if (rc != GZ_OK) {
     h->planes_mode = keep_mode;
     h->planes = keep_planes;
+    h->plain_planes = keep_plain;
     h->codes3 = keep_codes3;
     h->pipe = keep_pipe;
     h->tile_shift = keep[0];

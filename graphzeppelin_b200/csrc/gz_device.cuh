@@ -121,11 +121,12 @@ __device__ __forceinline__ uint32_t tail_lo32(uint64_t pm) {
   rrmxmx8_tail_pre(pm, lo, hi);
   return lo ^ __funnelshift_r(lo, hi, 28);
 }
-// Depth code of one column: min(depth, 15) where depth = ctz(hash | 1 << B); cap = 1 << min(B, 15).
-// For B <= 15 this is the depth itself (depth <= B); for B > 15 the code 15 stands for "15 or
-// more" and the exact depth is recomputed by depth_exact where it is needed.
+// Depth code of one column: min(depth, E) where depth = ctz(hash | 1 << B); cap = 1 << min(B, E).
+// For B <= E this is the depth itself (depth <= B); for B > E the code E stands for "E or more" and
+// the exact depth is recomputed by depth_exact where it is needed.
 __device__ __forceinline__ uint32_t depth_code(uint64_t pm, uint32_t cap) {
-  return __clz(__brev(tail_lo32(pm) | cap));
+  const uint32_t y = tail_lo32(pm) | cap;
+  return 31 - __clz(y & (0u - y));
 }
 // depth = ctz(hash | 1 << B), B <= 63, given the premixed input
 __device__ __forceinline__ uint32_t depth_exact(uint64_t pm, uint32_t B) {

@@ -38,7 +38,7 @@ enum EntryKind : uint8_t {
   kEntryCoded3 = 2,  // the same with 3-bit codes (column c in bits 3c .. 3c + 2; the payload from
                      // bit 3C): code 7 = "7 or more", recomputed where the entry is applied
 };
-constexpr uint32_t kDepthEscape = 15;  // depth code for "15 or more"
+constexpr uint32_t kDepthEscape = 11;  // depth code for "11 or more" (the planes' last row)
 constexpr uint32_t kDepthEscape3 = 7;  // 3-bit depth code for "7 or more"
 inline uint32_t neighbour_bits(uint32_t V) {
   uint32_t ubits = 1;
@@ -107,23 +107,31 @@ cudaError_t gutter_sort_scatter(int input, const void *d_in, uint64_t n, GutterG
 cudaError_t gutter_scatter_global(int input, const void *d_in, uint64_t n, GutterGeom g, int G,
                                   uint64_t *cursor, uint2 *entries, cudaStream_t s);
 
-// ---- coded entries and bucket planes (gz_planes.cu) ---------------------------------------
-// A vertex sketch is accumulated in shared memory as four planes of kPlaneRows rows x
-// kPlaneSlots 32-bit slots: slot c < C is column c, slot C the deterministic bucket (row 0).
-// Row d of a column holds depth d; the last row is scratch (depth codes at or above it are
-// handled in HBM). Plane A XORs (neighbour | 1 << 31) of the entries whose neighbour is above
-// the vertex, plane B of the others; planes GA and GB their checksums.
+// ---- bucket planes and coded entries (gz_planes.cu) ---------------------------------------
+// A vertex sketch is accumulated in shared memory as two planes of kPlaneRows rows x kPlaneSlots
+// slots of two words: slot c < C is column c, slot C the deterministic bucket (row 0); sketches of
+// more columns go in groups of kPlaneSlots slots. Row d of a column holds depth d; the last row
+// collects the depths from its own on (those are handled in HBM). Plane A XORs (neighbour |
+// 1 << 31) of the entries whose neighbour is above the vertex, plane B of the others, each with
+// the entries' checksums beside it.
 constexpr uint32_t kPlaneSlots = 32;
 constexpr uint32_t kPlaneRows = 12;
-constexpr uint32_t kPlaneMaxColumns = kPlaneSlots - 1;
+constexpr uint32_t kPlaneMaxColumns = kPlaneSlots - 1;  // columns of one group beside the deterministic slot
+constexpr uint32_t kPlaneMaxColumnsWide = 256;          // columns of the plain-entry update, in groups
 constexpr uint32_t kPlaneMaxTile = 32;     // vertices per shared-memory tile
 struct PlaneHash {
   uint32_t C, B;
-  uint64_t kcol[kPlaneMaxColumns];  // xxh3_premix(flip of column seed c)
+  uint64_t kcol[kPlaneSlots];       // xxh3_premix(flip of column seed c)
   uint64_t kchk;                    // xxh3_premix(flip of the checksum seed)
+};
+struct PlaneHashWide {
+  uint32_t C, B;
+  uint64_t kcol[kPlaneMaxColumnsWide + kPlaneSlots];
+  uint64_t kchk;
 };
 struct PlaneGeom {
   uint32_t V, C, B, sketch_words;
+  uint32_t groups;      // groups of kPlaneSlots slots: (C + 1) / kPlaneSlots, rounded up
   uint32_t tile_shift;  // W = 1 << tile_shift vertices per tile
   uint32_t ntiles;
   uint32_t bin_shift;   // gutter bin (>= tile_shift): a bin holds 1 << (bin - tile) tiles
@@ -131,8 +139,8 @@ struct PlaneGeom {
   uint32_t direct_max;  // a tile with fewer entries is updated in place in HBM
 };
 PlaneHash plane_hash(uint64_t seed, uint32_t C, uint32_t B);
-// Records per tile of the hash sort-scatter for this bin count (0: the bins do not fit).
-uint32_t hash_sort_tile(uint32_t nbins, size_t smem_budget);
+// Records per tile of the hash sort-scatter for this bin count and n records (0: the bins do not fit).
+uint32_t hash_sort_tile(uint32_t nbins, size_t smem_budget, uint64_t n);
 // Hash every record once (all C columns) and write its two coded endpoint entries,
 // counting-sorted by bin, to entries[base[b] + ...]; fill (nbins u32) starts at zero.
 // kind = kEntryCoded or kEntryCoded3.
@@ -146,6 +154,17 @@ cudaError_t plane_update(const PlaneGeom &g, const PlaneHash &ph, uint8_t *sketc
                          const uint8_t *gutter, const ChunkTable &chunks, const uint32_t *bin_off,
                          int nchunks, uint32_t *work_counter, uint32_t *status, int grid,
                          int threads, cudaStream_t s);
+// The same for plain entries, hashed where they are applied (any number of columns up to
+// kPlaneMaxColumnsWide, CameoSketch or CubeSketch), plane_threads(tile_shift) threads a CTA.
+int plane_threads(uint32_t tile_shift);
+PlaneHashWide plane_hash_wide(uint64_t seed, uint32_t C, uint32_t B);
+cudaError_t plane_update_plain(const PlaneGeom &g, bool cube, const PlaneHashWide &ph, uint8_t *sketches,
+                               const uint8_t *gutter, const ChunkTable &chunks, const uint32_t *bin_off,
+                               int nchunks, uint32_t *work_counter, cudaStream_t s);
+// Records XORed straight into both endpoints' sketches in HBM (sparse calls of CameoSketch with at
+// most kPlaneMaxColumns columns); flags and drops records naming a vertex >= V.
+cudaError_t direct_records(const void *d_rec, uint64_t n, uint32_t V, uint32_t sketch_words,
+                           const PlaneHash &ph, uint8_t *sketches, uint32_t *status, cudaStream_t s);
 // Register-only rate of the per-column hash of this ingest: premixed input XOR a premixed
 // column constant, rrmxmx tail, depth code (blocks x threads x iters x 8 hashes).
 cudaError_t plane_hash_peak(uint32_t iters, int blocks, int threads, uint64_t *out, cudaStream_t s);

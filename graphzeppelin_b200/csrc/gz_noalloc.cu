@@ -7,7 +7,7 @@
 // loops where cudaMalloc / cudaFree would synchronize the device and stall every other stream.
 // For them this entry point takes the caller's sketches and records (both already in device
 // memory) and allocates nothing: its scratch memory (gutter entries, bin counts and offsets,
-// hash constants, status words) lives in one fixed, file-scope device array that every GPU which
+// status words) lives in one fixed, file-scope device array that every GPU which
 // loads the library holds until the process exits.
 #include <cuda_runtime.h>
 
@@ -41,8 +41,7 @@ constexpr size_t kOffScanTmp = align256(kOffCursor + (size_t)kNoAllocMaxBins * 8
 constexpr size_t kOffTotal = align256(kOffScanTmp + 64 * 8);
 constexpr size_t kOffBinOff = align256(kOffTotal + 8);
 constexpr size_t kOffFill = align256(kOffBinOff + ((size_t)kNoAllocMaxBins + 1) * 4);
-constexpr size_t kOffFlip = align256(kOffFill + (size_t)kNoAllocMaxBins * 4);
-constexpr size_t kOffStatus = align256(kOffFlip + (kNoAllocMaxColumns + 1) * 8);
+constexpr size_t kOffStatus = align256(kOffFill + (size_t)kNoAllocMaxBins * 4);
 constexpr size_t kScratchBytes = align256(kOffStatus + 16);  // about 34 MiB
 
 // The scratch array. Host code must not use this name as a device address: the address comes
@@ -83,36 +82,6 @@ void noalloc_params(uint32_t V, double f, uint32_t &C, uint32_t &B) {
   const double num_samples_div = 1 - std::log2(2 - 0.8);
   const size_t s = (size_t)std::ceil(f * std::log2((double)V) / num_samples_div);
   C = (uint32_t)std::max<size_t>(18, s);
-}
-
-// Entries of the vertices past the last whole shared-memory tile ([tail_start, V), all inside
-// one gutter bin) are folded into the caller's sketches with global atomicXor.
-__global__ void k_noalloc_tail(uint32_t *sketches, const uint2 *entries, const uint32_t *bin_off,
-                               uint32_t bin, uint32_t tail_start, uint32_t sketch_words,
-                               uint32_t C, uint32_t B, const uint64_t *flip) {
-  const uint32_t b = bin_off[bin], e = bin_off[bin + 1];
-  const uint64_t flip_chk = flip[C];
-  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) {
-    const uint2 x = entries[i];
-    if (x.x < tail_start) continue;
-    const uint32_t lo = max(x.x, x.y), hi = min(x.x, x.y);
-    const uint64_t in64 = ((uint64_t)lo << 32) | hi;
-    const uint32_t chk = (uint32_t)gz::rrmxmx8(in64 ^ flip_chk);
-    uint32_t *sk = sketches + (uint64_t)x.x * sketch_words;
-    uint32_t *det = sk + 3 * C * B;
-    atomicXor(det, lo);
-    atomicXor(det + 1, hi);
-    atomicXor(det + 2, chk);
-    for (uint32_t c = 0; c < C; ++c) {
-      const uint32_t d = gz::depth_of(gz::rrmxmx8(in64 ^ flip[c]), B);
-      if (d < B) {
-        uint32_t *bk = sk + 3 * (c * B + d);
-        atomicXor(bk, lo);
-        atomicXor(bk + 1, hi);
-        atomicXor(bk + 2, chk);
-      }
-    }
-  }
 }
 
 #define NA_CUDA(call)                                                                     \
@@ -162,28 +131,22 @@ int gz_ingest_records_noalloc(void *d_sketches, uint32_t num_vertices, uint64_t 
   int rc = scratch_for_current_device(&scratch);
   if (rc != GZ_OK) return rc;
 
-  // geometry: the default tiling rule of the handle path
+  // tiles of 8 vertices with a gutter bin each; of 16 or 32 where that many more vertices still keep
+  // the bins within the shared-memory sort, or within the scratch's bins, with several tiles of 32 a
+  // bin past that
   const uint32_t nb = C * B + 1;
-  const uint64_t sketch_bytes = (uint64_t)nb * 12;
   int dev = 0, smem_optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (smem_optin <= 0) smem_optin = 227 * 1024;
-  const size_t budget = (size_t)smem_optin - 64 - gz::kQueueBytes;
-  const size_t flip_bytes = (size_t)(C + 1) * 8;
-  uint32_t shift = 2;
-  const uint64_t want = std::max<uint64_t>(4, num_vertices / (2ull * gz::num_sms()));
-  while (shift < 6 && (1ull << (shift + 1)) <= want && (sketch_bytes << (shift + 1)) + flip_bytes <= budget)
+  auto tiles_of = [&](uint32_t sh) { return (uint32_t)(((uint64_t)num_vertices + (1u << sh) - 1) >> sh); };
+  uint32_t shift = 3;
+  while (shift < 5 && (tiles_of(shift) > kNoAllocMaxBins ||
+                       (tiles_of(shift) > gz::kSortBinsMax && tiles_of(5) <= gz::kSortBinsMax)))
     ++shift;
-  if ((sketch_bytes << shift) + flip_bytes > budget)
-    return noalloc_fail(GZ_ERR_INVALID, "sketch too large to stage 4 vertices in shared memory");
   uint32_t bshift = shift;
-  while (((num_vertices + (1u << bshift) - 1) >> bshift) > 4096 && (1u << (bshift - shift)) < 16)
-    ++bshift;
-  const uint32_t nbins = (num_vertices + (1u << bshift) - 1) >> bshift;
-  if (nbins > kNoAllocMaxBins) return noalloc_fail(GZ_ERR_INVALID, "too many gutter bins");
-  const uint32_t full_tiles = num_vertices >> shift;
-  const uint32_t tail_start = full_tiles << shift;
+  while (tiles_of(bshift) > kNoAllocMaxBins) ++bshift;
+  const uint32_t nbins = tiles_of(bshift);
 
   // scratch regions
   uint2 *entries = reinterpret_cast<uint2 *>(scratch + kOffEntries);
@@ -193,15 +156,10 @@ int gz_ingest_records_noalloc(void *d_sketches, uint32_t num_vertices, uint64_t 
   uint64_t *total = reinterpret_cast<uint64_t *>(scratch + kOffTotal);
   uint32_t *bin_off = reinterpret_cast<uint32_t *>(scratch + kOffBinOff);
   uint32_t *fill = reinterpret_cast<uint32_t *>(scratch + kOffFill);
-  uint64_t *flip = reinterpret_cast<uint64_t *>(scratch + kOffFlip);
   uint32_t *status = reinterpret_cast<uint32_t *>(scratch + kOffStatus);  // [0] bits, [1] work
 
   // the array keeps the previous call's contents: reset what must start at zero
-  uint64_t hflip[kNoAllocMaxColumns + 1];
-  for (uint32_t c = 0; c < C; ++c) hflip[c] = gz::xxh3_flip(seed + 5ull * c);
-  hflip[C] = gz::xxh3_flip(seed);
   drain.armed = true;
-  NA_CUDA(cudaMemcpyAsync(flip, hflip, flip_bytes, cudaMemcpyHostToDevice, s));
   NA_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint64_t) * nbins, s));
   NA_CUDA(cudaMemsetAsync(fill, 0, sizeof(uint32_t) * nbins, s));
   NA_CUDA(cudaMemsetAsync(status, 0, 16, s));
@@ -221,32 +179,21 @@ int gz_ingest_records_noalloc(void *d_sketches, uint32_t num_vertices, uint64_t 
     NA_CUDA(gz::gutter_scatter_global(gz::kInputRecords, d_records, n_records, gg, G, cursor,
                                       entries, s));
   }
-  if (full_tiles) {
-    gz::SketchGeom g;
-    g.V = num_vertices;
-    g.C = C;
-    g.B = B;
-    g.sketch_words = nb * 3;
-    g.tile_shift = shift;
-    g.ntiles = full_tiles;  // whole tiles only: the tail never leaves the caller's buffer
-    g.bin_shift = bshift;
-    g.nbins = nbins;
-    NA_CUDA(gz::sketch_update_prepare(g, 1024));
-    gz::ChunkTable chunks{};
-    chunks.base[0] = 0;
-    chunks.kind[0] = gz::kEntryPlain;
-    const int grid = (int)std::min<uint64_t>(full_tiles, (uint64_t)gz::num_sms() *
-                                                             gz::sketch_update_ctas_per_sm(g, 1024));
-    NA_CUDA(gz::sketch_update(g, static_cast<uint8_t *>(d_sketches),
-                              reinterpret_cast<const uint8_t *>(entries), chunks, bin_off, 1, flip,
-                              status + 1, status, grid, 1024, s));
-  }
-  if (tail_start < num_vertices) {
-    k_noalloc_tail<<<std::max(1, gz::num_sms()), 256, 0, s>>>(
-        static_cast<uint32_t *>(d_sketches), entries, bin_off, tail_start >> bshift, tail_start,
-        nb * 3, C, B, flip);
-    NA_CUDA(cudaGetLastError());
-  }
+  gz::PlaneGeom g{};
+  g.V = num_vertices;
+  g.C = C;
+  g.B = B;
+  g.sketch_words = nb * 3;
+  g.groups = (C + gz::kPlaneSlots) / gz::kPlaneSlots;
+  g.tile_shift = shift;
+  g.ntiles = tiles_of(shift);
+  g.bin_shift = bshift;
+  g.nbins = nbins;
+  gz::ChunkTable chunks{};
+  chunks.base[0] = 0;
+  chunks.kind[0] = gz::kEntryPlain;
+  NA_CUDA(gz::plane_update_plain(g, false, gz::plane_hash_wide(seed, C, B), static_cast<uint8_t *>(d_sketches),
+                                 reinterpret_cast<const uint8_t *>(entries), chunks, bin_off, 1, status + 1, s));
   uint32_t st = 0;
   NA_CUDA(cudaMemcpyAsync(&st, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   NA_CUDA(cudaStreamSynchronize(s));

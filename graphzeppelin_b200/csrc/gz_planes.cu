@@ -23,9 +23,10 @@
 // applied, so the planes see the same 4-bit codes either way.
 //
 // Bucket planes. A warp takes 32 entries, one per lane. At step t = 0..31 lane l handles slot
-// l ^ t of its entry: slot c < C is column c, slot C the deterministic bucket, higher slots are
-// unused. A plane row is 32 words, so slot s is shared-memory bank s and the 32 lanes of a step hit
-// 32 different banks whatever their vertices and depths: the red.shared.xor never conflict (the
+// l ^ t of its entry: slot s < C is column s, slot C the deterministic bucket, higher slots are
+// unused (sketches of more columns go in groups of 32 slots, one pass over the entries each). A
+// plane row holds 32 slots, so slot s is shared-memory bank s and the 32 lanes of a step hit 32
+// different banks whatever their vertices and depths: the red.shared.xor never conflict (the
 // per-entry ordering, every lane on column c at once, concentrates lanes on a few banks because
 // depth 0 takes half the updates). Each bucket is kept as three words,
 //   A = XOR of (neighbour | 1 << 31) over the entries whose neighbour is above the vertex,
@@ -36,9 +37,16 @@
 //   alpha low  = low31(A) ^ (top bit of B ? vertex : 0),
 //   alpha high = low31(B) ^ (top bit of A ? vertex : 0),
 // the top bits holding the parity of each kind's entry count (vertex ids are below 2^31).
-// Rows hold depths 0 .. kPlaneRows - 2; the last row is scratch. Depths at or above it (2^-11 of
-// the column updates) are XORed into the sketch in HBM with global atomics; those rows are never
-// touched by the write-back, which rewrites only the rows the planes hold.
+// Rows hold depths 0 .. kPlaneRows - 2; the last row collects the depths at or above it (2^-11 of
+// the column updates), which are XORed into the sketch in HBM with global atomics; those rows are
+// never touched by the write-back, which changes only the rows the planes hold.
+//
+// What bounds the update: shared-memory issue. A slot step is two red.shared.xor, one wavefront
+// each, 64 wavefronts per 32 entries and SM. The address of a step is made by one byte permute
+// and one XOR: a row is 256 bytes -- 32 slots of A (or B), then the same slots' checksums, reached with
+// an immediate offset of 128 -- so that address byte 0 is the slot, byte 1 the row (the code plus the
+// plane's first row, added to four codes at once; planes never straddle a 64 KB boundary), and the
+// rest the plane's 64 KB block.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,36 +63,58 @@ namespace {
 
 using namespace gz::dev;
 
-constexpr uint32_t kPlaneThr = kPlaneRows - 1;               // first depth not held in the planes
-constexpr uint32_t kPlaneBytes = kPlaneRows * kPlaneSlots * 4;  // one plane of one vertex
-// Planes of one vertex: A, its checksums GA, B, its checksums GB. Each checksum plane sits one
-// plane after the plane it pairs with, so a slot step's second address is the first plus a
-// constant (an immediate of the reduction) whichever of A and B the entry goes to; the sketch's
-// checksum word is GA ^ GB.
-constexpr uint32_t kVertBytes = 4 * kPlaneBytes;
-constexpr uint32_t kQueueSlots = 64;                          // per-warp queue of filtered entries
-constexpr uint32_t kWbWords = kQueueSlots * 4;                // per-warp buffer: the entry queue
+constexpr uint32_t kPlaneThr = kPlaneRows - 1;  // first depth not held in the planes
+constexpr uint32_t kRowBytes = 256;             // 32 slots, then their checksums
+constexpr uint32_t kGOff = kPlaneSlots * 4;     // a slot's checksum sits this far behind it
+constexpr uint32_t kQueueSlots = 64;            // per-warp queue of filtered entries
 
-// Depth codes of all C columns into the nibble words w (column c in bits 4(c % 8) of word c / 8;
-// nibbles past C are zero); pm = premixed edge index. Every sketch has at least 18 columns: the
-// first 18 are unrolled, the rest a loop of exactly C - 18 steps.
-__device__ __forceinline__ void all_codes(uint64_t pm, const uint64_t *kcol, uint32_t C,
-                                          uint32_t cap, uint32_t (&w)[4]) {
-  w[0] = w[1] = 0;
-#pragma unroll
-  for (int c = 0; c < 16; ++c) w[c >> 3] |= depth_code(pm ^ kcol[c], cap) << (4 * (c & 7));
-  uint64_t hiw = (uint64_t)depth_code(pm ^ kcol[16], cap) |
-                 ((uint64_t)depth_code(pm ^ kcol[17], cap) << 4);
-#pragma unroll 2
-  for (uint32_t c = 18; c < C; ++c) hiw |= (uint64_t)depth_code(pm ^ kcol[c], cap) << (4 * (c - 16));
-  w[2] = (uint32_t)hiw;
-  w[3] = (uint32_t)(hiw >> 32);
+constexpr uint32_t kPairRows = 2 * kPlaneRows;  // planes A and B of one vertex, back to back
+
+// Bytes of the planes of 1 << tile_shift vertices, the unused rows before 64 KB boundaries included,
+// when they start within the first 4 KB of the block's shared memory: 10 pairs fit before the first
+// boundary and 10 between boundaries, and 4 KB at most are left over.
+__host__ __device__ constexpr uint32_t planes_bytes(uint32_t tile_shift) {
+  const uint32_t n = 1u << tile_shift;
+  return n * kPairRows * kRowBytes + (n - 1) / 10 * 4096u;
 }
 
-// Coded entry of vertex a (neighbour b): the codes, then from bit 4C the payload
-// (b << bin_shift) | (a & bin mask).
+// Depth codes of up to 32 columns into the nibble words w (column c of kcol in bits 4 (c % 8) of
+// word c / 8; nibbles past nc are zero); pm = premixed edge index. min(depth, 11) of a hash is the
+// place of the lowest bit of (hash | cap), 31 - clz of that bit alone (a quarter-rate bit reverse
+// less than counting trailing zeros: 1.48e12 against 1.34e12 codes/s on a register-only kernel).
+// The clz values, 16 .. 31 each, are summed at nibble distances; taking 16 per nibble off and
+// complementing turns all of a word's nibbles into codes at once. LO columns are known to exist.
+template <int LO>
+__device__ __forceinline__ void all_codes(uint64_t pm, const uint64_t *kcol, uint32_t nc, uint32_t cap,
+                                          uint32_t (&w)[4]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t x = 0;
+    if (8 * q < LO || 8u * q < nc) {
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        const int c = 8 * q + k;
+        if (c + 1 < LO || (uint32_t)c < nc) {
+          const uint32_t y0 = tail_lo32(pm ^ kcol[c]) | cap, y1 = tail_lo32(pm ^ kcol[c + 1]) | cap;
+          x += (uint32_t)__clz(y0 & (0u - y0)) << (4 * k);
+          x += (uint32_t)__clz(y1 & (0u - y1)) << (4 * k + 4);
+        }
+      }
+      x = ~(x - 0x11111110u);
+      const uint32_t n = 8 * q + 8 <= LO ? 8u : min(nc - 8u * q, 8u);
+      if (8 * q + 8 > LO && n < 8) x &= (1u << (4 * n)) - 1u;
+    }
+    w[q] = x;
+  }
+}
+
+// Coded entry of vertex a (neighbour b): the codes, then the payload (b << bin_shift) | (a & bin
+// mask): in the last word where the codes leave it free (every sketch up to 2^17 vertices; taking
+// an entry apart then needs no 64-bit shifts), else from bit 4C on.
+constexpr uint32_t kWordCodes = 24;  // columns whose codes leave the last word free
 __device__ __forceinline__ uint4 pack_entry(const uint32_t (&w)[4], uint32_t a, uint32_t b,
                                             uint32_t C, uint32_t bin_shift) {
+  if (C <= kWordCodes) return make_uint4(w[0], w[1], w[2], (b << bin_shift) | (a & ((1u << bin_shift) - 1u)));
   const uint64_t pay = ((uint64_t)b << bin_shift) | (a & ((1u << bin_shift) - 1u));
   const uint64_t hi = (((uint64_t)w[3] << 32) | w[2]) | (pay << (4 * C - 64));
   return make_uint4(w[0], w[1], (uint32_t)hi, (uint32_t)(hi >> 32));
@@ -93,6 +123,15 @@ __device__ __forceinline__ uint4 pack_entry(const uint32_t (&w)[4], uint32_t a, 
 // Vertex, neighbour and codes of a coded entry lying in gutter bin `bin`.
 __device__ __forceinline__ void unpack_entry(uint4 e, uint32_t bin, uint32_t C, uint32_t bin_shift,
                                              uint32_t &v, uint32_t &u, uint32_t (&w)[4]) {
+  if (C <= kWordCodes) {
+    v = (bin << bin_shift) | (e.w & ((1u << bin_shift) - 1u));
+    u = e.w >> bin_shift;
+    w[0] = e.x;
+    w[1] = e.y;
+    w[2] = e.z;
+    w[3] = 0;
+    return;
+  }
   const uint64_t hi = ((uint64_t)e.w << 32) | e.z;
   const uint32_t sh = 4 * C - 64;
   const uint64_t pay = hi >> sh;
@@ -165,7 +204,7 @@ __device__ __forceinline__ void unpack_entry3(uint4 e, uint32_t bin, uint32_t C,
 }
 
 // The 4-bit codes of a 3-bit coded entry: every escaped column (code 7: depth 7 or more) hashed
-// again for min(depth, 15). Out of line: about one entry in five at 28 columns has an escape.
+// again for min(depth, 11). Out of line: about one entry in five at 28 columns has an escape.
 __device__ __noinline__ uint4 fix_escapes3(uint4 w4, uint64_t pm, const uint64_t *kcol, uint32_t cap) {
   uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
@@ -288,7 +327,7 @@ k_hash_sort_scatter(const uint8_t *__restrict__ rec, uint64_t n, GutterGeom g, P
         const uint32_t lo = max(ru[k], rv[k]), hi = min(ru[k], rv[k]);
         const uint64_t pm = xxh3_premix(((uint64_t)lo << 32) | hi);
         uint32_t w[4];
-        all_codes(pm, ph.kcol, ph.C, cap, w);
+        all_codes<18>(pm, ph.kcol, ph.C, cap, w);
         s_ent[pu[k]] = C3 ? pack_entry3(w, ru[k], rv[k], ph.C, g.bin_shift)
                           : pack_entry(w, ru[k], rv[k], ph.C, g.bin_shift);
         s_ent[pv[k]] = C3 ? pack_entry3(w, rv[k], ru[k], ph.C, g.bin_shift)
@@ -307,30 +346,40 @@ k_hash_sort_scatter(const uint8_t *__restrict__ rec, uint64_t n, GutterGeom g, P
 // ------------------------------------------------------------------------------------------------
 // bucket-plane sketch update
 // ------------------------------------------------------------------------------------------------
+// (No memory clobber: the planes are touched by assembly alone, ordered by its volatility and the CTA
+// barriers, and other loads may move across.)
 __device__ __forceinline__ void red_xor_shared(uint32_t addr, uint32_t v) {
-  asm volatile("red.shared.xor.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+  asm volatile("red.shared.xor.b32 [%0], %1;" ::"r"(addr), "r"(v));
 }
-// The same slot of the checksum plane that follows the plane of addr.
+// The same slot's checksum.
 __device__ __forceinline__ void red_xor_shared_g(uint32_t addr, uint32_t v) {
-  asm volatile("red.shared.xor.b32 [%0+%2], %1;" ::"r"(addr), "r"(v), "n"(kPlaneBytes) : "memory");
+  asm volatile("red.shared.xor.b32 [%0+%2], %1;" ::"r"(addr), "r"(v), "n"(kGOff));
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
 }
 
-__device__ __forceinline__ uint32_t nibble_of(const uint32_t (&c4)[4], uint32_t c) {
-  const uint32_t w = c < 16 ? (c < 8 ? c4[0] : c4[1]) : (c < 24 ? c4[2] : c4[3]);
-  return (w >> (4 * (c & 7))) & 15u;
+// First row (shared-memory address / 256) of the planes of vertex vl of a tile whose planes start at
+// row r0: pairs of planes back to back, none across a 64 KB boundary.
+__device__ __forceinline__ uint32_t pair_row(uint32_t r0, uint32_t vl) {
+  uint32_t r = r0;
+  for (;;) {
+    const uint32_t fit = (256u - (r & 255u)) / kPairRows;  // pairs before the boundary
+    if (vl < fit) return r + vl * kPairRows;
+    vl -= fit;
+    r = (r | 255u) + 1;
+  }
 }
 
-// Flags of the codes at or above the scratch row: per word, bit 4 of byte lane j flags nibble 2j
-// and bit 5 flags nibble 2j + 1 (for a nibble n < 16, n + 5 carries into bit 4 of its byte lane
-// exactly when n >= 11).
-__device__ __forceinline__ uint32_t high_code_flags(uint32_t w) {
-  static_assert(kPlaneThr == 11, "the byte-lane test below is written for threshold 11");
-  const uint32_t lo = ((w & 0x0f0f0f0fu) + 0x05050505u) & 0x10101010u;
-  const uint32_t hi = ((((w >> 4) & 0x0f0f0f0fu) + 0x05050505u) & 0x10101010u) << 1;
-  return lo | hi;
+// Bits 4n + 3 of the nibbles n holding the escape code (codes do not exceed it).
+__device__ __forceinline__ uint32_t deep_codes(uint32_t w) {
+  static_assert(kDepthEscape == 11 && kDepthEscape == kPlaneThr, "11: bits 3, 1 and 0; the last plane row");
+  return w & (w << 2) & (w << 3) & 0x88888888u;
 }
 
-// Bucket (c, d) of vertex v's sketch in HBM, three 32-bit atomics (alpha low, alpha high, gamma).
+// Bucket of a sketch in HBM, three 32-bit atomics (alpha low, alpha high, gamma).
 __device__ __forceinline__ void xor_bucket_global(uint32_t *sk, uint32_t bucket, uint32_t lo,
                                                   uint32_t hi, uint32_t chk) {
   uint32_t *p = sk + 3 * bucket;
@@ -339,42 +388,41 @@ __device__ __forceinline__ void xor_bucket_global(uint32_t *sk, uint32_t bucket,
   atomicXor(p + 2, chk);
 }
 
-// Moves the codes at or above the scratch row into HBM (exact depth; code 15 means 15 or more
-// and is recomputed) and points them at the scratch row. Rare per column (2^-11), so only the
-// flagged nibbles are visited.
-__device__ __noinline__ uint4 spill_high_codes(uint4 cw, uint4 fl, uint64_t pm, uint32_t lo,
-                                               uint32_t hi, uint32_t chk, uint32_t *sk,
-                                               const uint64_t *s_kcol, uint32_t B) {
-  uint32_t c4[4] = {cw.x, cw.y, cw.z, cw.w};
-  const uint32_t f4[4] = {fl.x, fl.y, fl.z, fl.w};
-#pragma unroll
+// The columns of an entry whose code is the escape (depth 11 or more): XORed into HBM at their exact
+// depth (CubeSketch: at every depth from the last row's on). They went to the planes' last row,
+// which CubeSketch needs to hold exactly the depths below B: a depth of B is taken out of it again
+// (last_row: address of slot 0 of that row). kcol and c0: the group's columns.
+template <bool CUBE>
+__device__ __forceinline__ void apply_deep(const uint32_t (&c4)[4], uint64_t pm, uint32_t v, uint32_t u,
+                                           uint32_t chk, uint32_t *sk, const uint64_t *kcol, uint32_t c0,
+                                           uint32_t B, uint32_t last_row) {
+  const uint32_t lo = max(u, v), hi = min(u, v);
+#pragma unroll 1
   for (int w = 0; w < 4; ++w) {
-    uint32_t f = f4[w];
-    while (f) {
-      const uint32_t bit = __ffs(f) - 1;  // 4 + 8j (nibble 2j) or 5 + 8j (nibble 2j + 1)
-      f &= f - 1;
-      const uint32_t nib = 2 * (bit >> 3) + (bit & 1u);  // nibble inside the word
-      const uint32_t c = 8 * w + nib, sh = 4 * nib;
-      const uint32_t code = (c4[w] >> sh) & 15u;
-      const uint32_t d = code < kDepthEscape ? code : depth_exact(pm ^ s_kcol[c], B);
-      if (d < B) xor_bucket_global(sk, c * B + d, lo, hi, chk);
-      c4[w] = (c4[w] & ~(15u << sh)) | (kPlaneThr << sh);
+    for (uint32_t f = deep_codes(w == 0 ? c4[0] : w == 1 ? c4[1] : w == 2 ? c4[2] : c4[3]); f; f &= f - 1) {
+      const uint32_t c = 8 * w + ((__ffs(f) - 1) >> 2);
+      const uint32_t d = depth_exact(pm ^ kcol[c], B);
+      if (CUBE) {
+        if (d < B) {
+          for (uint32_t j = kPlaneThr; j <= d; ++j) xor_bucket_global(sk, (c0 + c) * B + j, lo, hi, chk);
+        } else {
+          red_xor_shared(last_row + 4 * c, u | 0x80000000u);
+          red_xor_shared_g(last_row + 4 * c, chk);
+        }
+      } else if (d < B) {
+        xor_bucket_global(sk, (c0 + c) * B + d, lo, hi, chk);
+      }
     }
   }
-  return make_uint4(c4[0], c4[1], c4[2], c4[3]);
 }
 
-// nibble t of the result = nibble t ^ lane of the input (5 index bits: half-byte, byte pair in
-// the word, word)
+// nibble t of the result = nibble t ^ (lane & 30) of the input (byte in the word, word; the lowest
+// index bit is taken where the nibbles are widened)
 __device__ __forceinline__ void permute_codes(uint32_t (&c4)[4], uint32_t lane) {
-  if (lane & 1) {
-#pragma unroll
-    for (int w = 0; w < 4; ++w) c4[w] = ((c4[w] >> 4) & 0x0f0f0f0fu) | ((c4[w] & 0x0f0f0f0fu) << 4);
-  }
   const uint32_t q = (lane >> 1) & 3u;
   const uint32_t sel = q | ((1u ^ q) << 4) | ((2u ^ q) << 8) | ((3u ^ q) << 12);
 #pragma unroll
-  for (int w = 0; w < 4; ++w) c4[w] = __byte_perm(c4[w], 0, sel);
+  for (int w = 0; w < 4; ++w) c4[w] = prmt(c4[w], 0, sel);
   if (lane & 8) {
     uint32_t x = c4[0]; c4[0] = c4[1]; c4[1] = x;
     x = c4[2]; c4[2] = c4[3]; c4[3] = x;
@@ -385,307 +433,439 @@ __device__ __forceinline__ void permute_codes(uint32_t (&c4)[4], uint32_t lane) 
   }
 }
 
-struct PlaneCtx {
-  uint32_t sp, tile_mask, sketch_words, C, B, cap, bin_shift;
-  uint32_t *gsk;
-  const uint64_t *s_kcol;
-  uint64_t kchk;
-};
-
-// All codes of a plain {vertex, neighbour} entry (apply_update_batch), hashed where it is applied;
-// out of line, so the coded path keeps its registers.
-__device__ __noinline__ uint4 plain_codes(uint64_t pm, const uint64_t *kcol, uint32_t C, uint32_t cap) {
-  uint32_t w[4];
-  all_codes(pm, kcol, C, cap, w);
-  return make_uint4(w[0], w[1], w[2], w[3]);
+// The 32 slot steps of one entry per lane: codes c4 (already permuted), plane starting at row `row`.
+__device__ __forceinline__ void slot_steps(const uint32_t (&c4)[4], uint32_t row, uint32_t val,
+                                           uint32_t chk, uint32_t lane) {
+  const uint32_t radd = (row & 255u) * 0x01010101u;
+  const uint32_t base = ((row >> 8) << 16) | (lane << 2), odd = 4 * (lane & 1);
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    // one byte per step: the row inside the plane's 64 KB block
+    const uint32_t ev = ((c4[w] >> odd) & 0x0f0f0f0fu) + radd, od = ((c4[w] >> (4 - odd)) & 0x0f0f0f0fu) + radd;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t t = 8 * w + j;
+      // byte 1: the row; byte 0: the slot; the plane's block
+      const uint32_t a = prmt((j & 1) ? od : ev, base ^ (t << 2), 0x7604u | ((uint32_t)(j >> 1) << 4));
+      red_xor_shared(a, val);
+      red_xor_shared_g(a, chk);
+    }
+  }
 }
 
-// Vertex, neighbour and 4-bit codes of a gutter entry (kind) of bin `bin`: unpacked from a coded
-// entry (3-bit codes: escapes hashed again), or hashed here for a plain {vertex, neighbour} entry
-// (apply_update_batch).
-__device__ __forceinline__ void decode_entry(uint4 e, uint32_t kind, uint32_t bin, const PlaneCtx &x,
-                                             uint32_t &v, uint32_t &u, uint64_t &pm, uint32_t (&c4)[4]) {
-  if (kind == kEntryCoded) {
-    unpack_entry(e, bin, x.C, x.bin_shift, v, u, c4);
-  } else if (kind == kEntryCoded3) {
-    unpack_entry3(e, bin, x.C, x.bin_shift, v, u, c4);
+// Vertex, neighbour, premixed index and codes (of the group's nc columns, constants kcol) of a gutter
+// entry of bin `bin`: unpacked from a coded entry (3-bit codes: escapes hashed again), or hashed here
+// for a plain {vertex, neighbour} entry.
+template <int KIND>
+__device__ __forceinline__ void decode_entry(uint4 e, uint32_t bin, const PlaneGeom &g, uint32_t cap,
+                                             const uint64_t *kcol, uint32_t nc, uint32_t &v, uint32_t &u,
+                                             uint64_t &pm, uint32_t (&c4)[4]) {
+  if (KIND == kEntryCoded) {
+    unpack_entry(e, bin, g.C, g.bin_shift, v, u, c4);
+  } else if (KIND == kEntryCoded3) {
+    unpack_entry3(e, bin, g.C, g.bin_shift, v, u, c4);
   } else {
     v = e.x;
     u = e.y;
   }
   pm = xxh3_premix(((uint64_t)max(u, v) << 32) | min(u, v));  // idx = (min << 32) | max
-  if (kind == kEntryCoded3) {
+  if (KIND == kEntryCoded3) {
     const uint32_t esc = ((c4[0] + 0x11111111u) | (c4[1] + 0x11111111u) | (c4[2] + 0x11111111u) |
                           (c4[3] + 0x11111111u)) & 0x88888888u;
     if (esc) {
-      const uint4 w = fix_escapes3(make_uint4(c4[0], c4[1], c4[2], c4[3]), pm, x.s_kcol, x.cap);
+      const uint4 w = fix_escapes3(make_uint4(c4[0], c4[1], c4[2], c4[3]), pm, kcol, cap);
       c4[0] = w.x;
       c4[1] = w.y;
       c4[2] = w.z;
       c4[3] = w.w;
     }
-  } else if (kind == kEntryPlain) {
-    const uint4 w = plain_codes(pm, x.s_kcol, x.C, x.cap);
-    c4[0] = w.x;
-    c4[1] = w.y;
-    c4[2] = w.z;
-    c4[3] = w.w;
+  } else if (KIND == kEntryPlain) {
+    all_codes<0>(pm, kcol, nc, cap, c4);
   }
 }
 
 // Vertex of a gutter entry of bin `bin` (for filtering a bin's entries by tile).
-__device__ __forceinline__ uint32_t entry_vertex(uint4 e, uint32_t kind, uint32_t bin, const PlaneCtx &x) {
-  if (kind == kEntryPlain) return e.x;
-  const uint64_t pay = kind == kEntryCoded3 ? payload3(e, x.C)
-                                            : (((uint64_t)e.w << 32) | e.z) >> (4 * x.C - 64);
-  return (bin << x.bin_shift) | ((uint32_t)pay & ((1u << x.bin_shift) - 1u));
+template <int KIND>
+__device__ __forceinline__ uint32_t entry_vertex(uint4 e, uint32_t bin, const PlaneGeom &g) {
+  if (KIND == kEntryPlain) return e.x;
+  if (KIND == kEntryCoded && g.C <= kWordCodes) return (bin << g.bin_shift) | (e.w & ((1u << g.bin_shift) - 1u));
+  const uint64_t pay = KIND == kEntryCoded3 ? payload3(e, g.C)
+                                            : (((uint64_t)e.w << 32) | e.z) >> (4 * g.C - 64);
+  return (bin << g.bin_shift) | ((uint32_t)pay & ((1u << g.bin_shift) - 1u));
 }
 
-// One entry per lane into the tile's planes (invalid lanes XOR zeros into vertex 0 of the tile).
-__device__ __forceinline__ void plane_entry(uint4 e, uint32_t kind, bool valid, uint32_t bin,
-                                            uint32_t lane, const PlaneCtx &x) {
-  uint32_t v, u, c4[4];
-  uint64_t pm;
-  decode_entry(e, kind, bin, x, v, u, pm, c4);
-  const uint32_t lo = max(u, v), hi = min(u, v);
-  const uint32_t chk = valid ? tail_lo32(pm ^ x.kchk) : 0u;
-  const uint32_t val = valid ? (u | 0x80000000u) : 0u;
-  const uint32_t p = u > v ? 0u : 1u;  // plane A or B
-  if (!valid) c4[0] = c4[1] = c4[2] = c4[3] = 0;
-  const uint4 fl = make_uint4(high_code_flags(c4[0]), high_code_flags(c4[1]), high_code_flags(c4[2]),
-                              high_code_flags(c4[3]));
-  if (fl.x | fl.y | fl.z | fl.w) {
-    const uint4 y = spill_high_codes(make_uint4(c4[0], c4[1], c4[2], c4[3]), fl, pm, lo, hi, chk,
-                                     x.gsk + (uint64_t)v * x.sketch_words, x.s_kcol, x.B);
-    c4[0] = y.x;
-    c4[1] = y.y;
-    c4[2] = y.z;
-    c4[3] = y.w;
-  }
-  permute_codes(c4, lane);
-  // one byte per step: byte k of ev[w] (od[w]) = 8 x code of nibble 2k (2k + 1) of word w, so a
-  // step takes its row offset with one byte extract
-  uint32_t ev[4], od[4];
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    ev[w] = (c4[w] & 0x0f0f0f0fu) << 3;
-    od[w] = ((c4[w] >> 4) & 0x0f0f0f0fu) << 3;
-  }
-  // bits 2..6 of base are the lane (sp is 128-byte aligned, the rest multiples of 128), and the
-  // row offset (a multiple of 128) leaves them alone, so (base + row) ^ (t << 2) addresses slot
-  // lane ^ t of the row
-  const uint32_t base = x.sp + (v & x.tile_mask) * kVertBytes + p * 2 * kPlaneBytes + (lane << 2);
-#pragma unroll
-  for (int t = 0; t < 32; ++t) {
-    const uint32_t w = (uint32_t)t >> 3, k = ((uint32_t)t & 7u) >> 1;
-    const uint32_t d8 = __byte_perm((t & 1) ? od[w] : ev[w], 0, 0x4440u + k);
-    const uint32_t a = (base + d8 * 16u) ^ (uint32_t)(t << 2);
-    red_xor_shared(a, val);
-    red_xor_shared_g(a, chk);
-  }
-}
-
-// One entry applied straight to HBM (sparse tiles): deterministic bucket, then each column.
-__device__ __forceinline__ void entry_in_place(uint4 e, uint32_t kind, uint32_t bin, uint32_t tile,
-                                               uint32_t tile_shift, const PlaneCtx &x) {
-  uint32_t v, u, c4[4];
-  uint64_t pm;
-  decode_entry(e, kind, bin, x, v, u, pm, c4);
-  if ((v >> tile_shift) != tile) return;
-  const uint32_t lo = max(u, v), hi = min(u, v);
-  const uint32_t chk = tail_lo32(pm ^ x.kchk);
-  uint32_t *sk = x.gsk + (uint64_t)v * x.sketch_words;
-  xor_bucket_global(sk, x.C * x.B, lo, hi, chk);
-  for (uint32_t c = 0; c < x.C; ++c) {
-    const uint32_t code = nibble_of(c4, c);
-    const uint32_t d = code < kDepthEscape ? code : depth_exact(pm ^ x.s_kcol[c], x.B);
-    if (d < x.B) xor_bucket_global(sk, c * x.B + d, lo, hi, chk);
-  }
-}
-
-__device__ __forceinline__ uint4 load_entry(const uint8_t *cb, uint32_t kind, uint32_t i) {
-  if (kind != kEntryPlain) return reinterpret_cast<const uint4 *>(cb)[i];
+template <int KIND>
+__device__ __forceinline__ uint4 load_entry(const uint8_t *cb, uint32_t i) {
+  if (KIND != kEntryPlain) return reinterpret_cast<const uint4 *>(cb)[i];
   const uint2 k = reinterpret_cast<const uint2 *>(cb)[i];
   return make_uint4(k.x, k.y, 0, 0);
 }
 
+// What a CTA works on: one group of columns of one tile.
+struct PlaneItem {
+  uint32_t t, bin, c0, nc;  // tile, its bin, the group's first column and number of columns
+  const uint64_t *kcol;     // the group's hash constants
+  uint32_t *gsk;
+  const uint32_t *row_of;   // first row of each vertex's planes
+  uint32_t *deep;           // bit l of word j: entry 32 j + l of the segment has an escape code
+};
+// Entries are taken in segments of 64 groups of 32 a warp; each warp looks at the escapes among its entries of
+// a segment (about 1 entry in 85 at 24 columns) together, after its last slot step.
+__host__ __device__ constexpr uint32_t deep_words(uint32_t threads) { return 2 * threads; }
+
+// An entry ready for its slot steps.
+struct Ready {
+  uint32_t c4[4], row, val, chk;
+};
+
+template <int KIND>
+__device__ __forceinline__ Ready ready_entry(uint4 en, const PlaneItem &x, const PlaneGeom &g, uint64_t kchk,
+                                             uint32_t cap, uint32_t tile_mask, uint32_t lane, bool &deep) {
+  Ready r;
+  uint32_t v, u;
+  uint64_t pm;
+  decode_entry<KIND>(en, x.bin, g, cap, x.kcol, x.nc, v, u, pm, r.c4);
+  r.chk = tail_lo32(pm ^ kchk);
+  r.val = u | 0x80000000u;
+  r.row = x.row_of[v & tile_mask] + (u > v ? 0u : kPlaneRows);  // plane A or B
+  deep = (deep_codes(r.c4[0]) | deep_codes(r.c4[1]) | deep_codes(r.c4[2]) | deep_codes(r.c4[3])) != 0;
+  permute_codes(r.c4, lane);
+  return r;
+}
+
+// Entries [b, e) of one gutter chunk (at cb; at most 32 deep_words(threads) of them) into the planes of the
+// item's tile.
+template <int KIND, bool CUBE>
+__device__ __forceinline__ void plane_chunk(const PlaneItem &x, const PlaneGeom &g, uint64_t kchk, uint32_t cap,
+                                            const uint8_t *cb, uint32_t b, uint32_t e, uint32_t *queue) {
+  const uint32_t nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t tile_mask = (1u << g.tile_shift) - 1, step = nwarps * 32;
+  // word j of this warp's escape mask: bit l of word warp + j nwarps, entry b + 32 word + l
+  auto deep_entries = [&]() {
+    __syncwarp();
+    for (uint32_t j = warp + lane * nwarps; j < (e - b + 31) / 32; j += step)
+      for (uint32_t m = x.deep[j]; m; m &= m - 1) {
+        uint32_t v, u, c4[4];
+        uint64_t pm;
+        decode_entry<KIND>(load_entry<KIND>(cb, b + 32 * j + __ffs(m) - 1), x.bin, g, cap, x.kcol, x.nc, v, u, pm,
+                           c4);
+        if ((v >> g.tile_shift) != x.t) continue;
+        const uint32_t row = x.row_of[v & tile_mask] + (u > v ? 0u : kPlaneRows);
+        apply_deep<CUBE>(c4, pm, v, u, tail_lo32(pm ^ kchk), x.gsk + (uint64_t)v * g.sketch_words, x.kcol, x.c0,
+                         g.B, (row + kPlaneThr) * kRowBytes);
+      }
+    __syncwarp();
+  };
+  if (g.bin_shift == g.tile_shift) {
+    // the bin is this tile: every entry applies. A warp's slot steps of one group of 32 entries (LSU)
+    // are issued between the arithmetic that makes the next group ready (ALU), and the group after
+    // that is being loaded. Lanes past the end repeat the last entry with nothing to XOR.
+    uint32_t i = b + warp * 32 + lane;
+    if (i - lane >= e) return;
+    uint32_t word = warp;
+    bool deep, any = false;
+    auto load = [&](uint32_t k) { return load_entry<KIND>(cb, min(k, e - 1)); };
+    uint4 nx = load(i);
+    Ready r = ready_entry<KIND>(nx, x, g, kchk, cap, tile_mask, lane, deep);
+    nx = load(i + step);
+    for (;; i += step, word += nwarps) {
+      const uint32_t m = __ballot_sync(kFull, deep && i < e);
+      if (lane == 0) x.deep[word] = m;
+      any = any || m;
+      if (i - lane + step >= e) break;
+      const Ready q = r;
+      r = ready_entry<KIND>(nx, x, g, kchk, cap, tile_mask, lane, deep);
+      nx = load(i + 2 * step);
+      slot_steps(q.c4, q.row, q.val, q.chk, lane);
+    }
+    const bool in = i < e;
+    slot_steps(r.c4, r.row, in ? r.val : 0u, in ? r.chk : 0u, lane);
+    if (any) deep_entries();
+  } else {
+    // the bin holds several tiles: each warp ballots its group, queues the indices of this tile's
+    // entries, and applies full warps of queued ones; two groups are in flight ahead of the one
+    // ballotted. The escape mask has the word of the group that an entry was found in.
+    uint32_t i0 = b + warp * 32, qn = 0;
+    for (uint32_t j = warp + lane * nwarps; j < (e - b + 31) / 32; j += step) x.deep[j] = 0;
+    __syncwarp();
+    bool any = false;
+    auto apply = [&](uint32_t i, bool valid) {
+      bool deep;
+      const Ready r = ready_entry<KIND>(load_entry<KIND>(cb, i), x, g, kchk, cap, tile_mask, lane, deep);
+      if (valid && deep) atomicOr(&x.deep[(i - b) >> 5], 1u << ((i - b) & 31));
+      any = __any_sync(kFull, any || (valid && deep));
+      slot_steps(r.c4, r.row, valid ? r.val : 0u, valid ? r.chk : 0u, lane);
+    };
+    auto tile_at = [&](uint32_t i) {
+      return i < e ? entry_vertex<KIND>(load_entry<KIND>(cb, i), x.bin, g) >> g.tile_shift : ~x.t;
+    };
+    uint32_t nx = tile_at(i0 + lane), nx2 = tile_at(i0 + step + lane);
+    for (; i0 < e; i0 += step) {
+      const bool mine = nx == x.t;
+      nx = nx2;
+      nx2 = tile_at(i0 + 2 * step + lane);
+      const uint32_t m = __ballot_sync(kFull, mine);
+      if (mine) queue[qn + __popc(m & ((1u << lane) - 1u))] = i0 + lane;
+      qn += __popc(m);
+      __syncwarp();
+      if (qn >= 32) {
+        const uint32_t q = queue[lane];
+        __syncwarp();
+        qn -= 32;
+        if (lane < qn) queue[lane] = queue[32 + lane];
+        __syncwarp();
+        apply(q, true);
+      }
+    }
+    if (qn) {
+      const uint32_t q = queue[lane < qn ? lane : 0];
+      __syncwarp();
+      apply(q, lane < qn);
+    }
+    if (any) deep_entries();
+  }
+}
+
+// One endpoint update XORed into the sketch sk in HBM by a whole warp: lane l < nc holds the depth
+// of column l (nothing to do when it is B or more), lane nc stands for the deterministic bucket.
+// The buckets' words are dealt over the lanes three to a bucket, so a bucket is one request to L2
+// instead of three.
+__device__ __forceinline__ void warp_update_global(uint32_t *sk, uint32_t nc, uint32_t depth,
+                                                   uint32_t B, uint32_t lo, uint32_t hi, uint32_t chk) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t off = lane < nc ? (depth < B ? 3 * (lane * B + depth) : 0xffffffffu) : 3 * nc * B;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const uint32_t f = i * 32 + lane, bk = f / 3, kk = f - 3 * bk;
+    const uint32_t o = __shfl_sync(kFull, off, bk);
+    if (bk <= nc && o != 0xffffffffu) atomicXor(sk + o + kk, kk == 0 ? lo : kk == 1 ? hi : chk);
+  }
+}
+
+// Sparse calls (few updates for the graph's size): every record hashed once, a warp per record and
+// a lane per column, and XORed into both endpoints' sketches in HBM: one launch, no gutter.
+// (A self-loop XORs one sketch twice: no change, as through the gutter.)
+__global__ void __launch_bounds__(256)
+k_direct_records(const uint8_t *__restrict__ rec, uint64_t n, uint32_t V, uint32_t sketch_words,
+                 PlaneHash ph, uint32_t *__restrict__ sk, uint32_t *__restrict__ status) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint64_t kc = lane < ph.C ? ph.kcol[lane] : ph.kchk;
+  for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
+    uint32_t u, v;
+    load_record(rec, rec + 9 * n, i, u, v);
+    if (u >= V || v >= V) {
+      if (lane == 0) atomicOr(status, kStatusBadVertex);
+      continue;
+    }
+    if (u == v) continue;
+    const uint32_t lo = max(u, v), hi = min(u, v);
+    const uint64_t pm = xxh3_premix(((uint64_t)lo << 32) | hi);
+    const uint32_t depth = depth_exact(pm ^ kc, ph.B);
+    const uint32_t chk = tail_lo32(pm ^ ph.kchk);
+    warp_update_global(sk + (uint64_t)u * sketch_words, ph.C, depth, ph.B, lo, hi, chk);
+    warp_update_global(sk + (uint64_t)v * sketch_words, ph.C, depth, ph.B, lo, hi, chk);
+  }
+}
+
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v));
+}
+
+// Write-back of one vertex's planes (A at shared address pa, B behind it) by one warp, and their
+// clearing for the next tile. col: the group's first column in the sketch; its nc columns start 3 B
+// words apart, and rows 0 .. R - 1 come from the planes, 3 R words a column; the deterministic bucket
+// is the first row of slot det (none in this group when det is 32 or more). Lane by column, a lane
+// turns its slot's rows into sketch words (every lane its own bank); the words are then laid down in
+// the order of the sketch over the planes themselves and taken in that order, so that the lanes read
+// and write consecutive words in HBM, 13 of them in flight per lane. Zero words are left alone.
+// (Global reductions instead run into L2's rate for them, about 45e9 sectors/s; reading the planes
+// in the order of the sketch is a 14-way bank conflict: 16 us a tile of 32 vertices.)
+template <bool CUBE>
+__device__ __forceinline__ void write_back(uint32_t pa, uint32_t vg, uint32_t *col, uint32_t nc, uint32_t det,
+                                           uint32_t B, uint32_t lane) {
+  constexpr uint32_t pb = kPlaneRows * kRowBytes;
+  const uint32_t R = min(B, kPlaneThr), run = 3 * R;
+  const uint32_t at = pa + 4 * lane;
+  const bool mine = lane < nc || lane == det;
+  uint32_t w[3 * kPlaneThr];
+  uint32_t s[4] = {0, 0, 0, 0};
+  if (CUBE && B > kPlaneThr) {  // the depths from kPlaneThr to B - 1
+    s[0] = lds32(at + kPlaneThr * kRowBytes);
+    s[1] = lds32(at + kPlaneThr * kRowBytes + kGOff);
+    s[2] = lds32(at + pb + kPlaneThr * kRowBytes);
+    s[3] = lds32(at + pb + kPlaneThr * kRowBytes + kGOff);
+  }
+#pragma unroll
+  for (int r = kPlaneThr - 1; r >= 0; --r) {
+    uint32_t a = 0, ga = 0, b = 0, gb = 0;
+    if (mine && (uint32_t)r < R) {
+      const uint32_t o = at + r * kRowBytes;
+      a = lds32(o);
+      ga = lds32(o + kGOff);
+      b = lds32(o + pb);
+      gb = lds32(o + pb + kGOff);
+    }
+    if (CUBE && lane != det) {
+      // CubeSketch: bucket d of a column takes every update of depth d or more
+      // (src/sketch.cpp:50-67), the suffix XOR over the rows
+      a = s[0] ^= a;
+      ga = s[1] ^= ga;
+      b = s[2] ^= b;
+      gb = s[3] ^= gb;
+    }
+    w[3 * r] = (a & 0x7fffffffu) ^ ((b >> 31) ? vg : 0u);
+    w[3 * r + 1] = (b & 0x7fffffffu) ^ ((a >> 31) ? vg : 0u);
+    w[3 * r + 2] = ga ^ gb;
+  }
+  __syncwarp();
+  const uint32_t list = nc * run + (det < 32 ? 3u : 0u);  // words; the deterministic bucket's last
+#pragma unroll
+  for (int i = 0; i < 3 * (int)kPlaneThr; ++i)
+    if ((lane < nc && (uint32_t)i < run) || (lane == det && i < 3)) sts32(pa + 4 * (lane * run + i), w[i]);
+  __syncwarp();
+  uint32_t c = 0, k = lane;  // word k of column c
+  while (k >= run) {
+    k -= run;
+    ++c;
+  }
+  for (uint32_t i0 = 0; i0 < list; i0 += 13 * 32) {
+    uint32_t y[13], old[13], off[13];
+#pragma unroll
+    for (int j = 0; j < 13; ++j) {
+      const uint32_t i = i0 + j * 32 + lane;
+      y[j] = i < list ? lds32(pa + 4 * i) : 0u;
+      off[j] = 3 * c * B + k;
+      old[j] = y[j] ? __ldcg(col + off[j]) : 0u;
+      k += 32;
+      while (k >= run) {
+        k -= run;
+        ++c;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 13; ++j)
+      if (y[j]) col[off[j]] = old[j] ^ y[j];
+  }
+  __syncwarp();
+#pragma unroll
+  for (uint32_t i = 0; i < kPairRows * kRowBytes / 512; ++i)
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(pa + i * 512 + lane * 16), "r"(0u));
+}
+
+// The update kernel: persistent CTAs take (tile, group) items. CODED: entries of the coded path
+// (sketches of one group of slots; plain entries come from apply_update_batch); otherwise plain
+// entries only, hashed here. Threads and tile size come with the launch: one CTA of 1024 threads and
+// 32 vertices per SM where the gutter's bins ask for large tiles; four of 256 threads and 8 vertices,
+// whose phases overlap each other, otherwise.
+template <bool CODED, bool CUBE, class Hash>
 __global__ void __launch_bounds__(1024, 1)
-k_plane_update(PlaneGeom g, PlaneHash ph, uint8_t *__restrict__ sketches,
-               const uint8_t *__restrict__ gutter, ChunkTable chunks,
-               const uint32_t *__restrict__ bin_off, int nchunks, uint32_t *work_counter) {
+k_plane_update(const __grid_constant__ PlaneGeom g, const __grid_constant__ Hash ph,
+               uint8_t *__restrict__ sketches, const uint8_t *__restrict__ gutter,
+               const __grid_constant__ ChunkTable chunks, const uint32_t *__restrict__ bin_off, int nchunks,
+               uint32_t *work_counter) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  __shared__ uint64_t s_kcol[kPlaneMaxColumns];
-  __shared__ uint32_t s_claim[2];
+  __shared__ uint32_t s_row[kPlaneMaxTile];
+  __shared__ uint32_t s_claim[2][2];
   const uint32_t W = 1u << g.tile_shift;
   const uint32_t nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t per_bin = g.bin_shift - g.tile_shift;  // log2(tiles per bin)
-  const uint32_t s0 = smem_u32(dsm);
-  const uint32_t pad = (128u - (s0 & 127u)) & 127u;
-  uint8_t *planes = dsm + pad;  // W vertices x planes A, GA, B, GB x kPlaneRows x 32 words
-  uint32_t *wbuf = reinterpret_cast<uint32_t *>(planes + (size_t)W * kVertBytes) + warp * kWbWords;
-  uint4 *queue = reinterpret_cast<uint4 *>(wbuf);  // the apply phase's per-warp entry queue
-  for (uint32_t i = threadIdx.x; i < g.C; i += blockDim.x) s_kcol[i] = ph.kcol[i];
-  PlaneCtx x;
-  x.sp = s0 + pad;
-  x.tile_mask = W - 1;
-  x.sketch_words = g.sketch_words;
-  x.C = g.C;
-  x.B = g.B;
-  x.cap = 1u << min(g.B, kDepthEscape);
-  x.bin_shift = g.bin_shift;
+  const uint32_t s0 = (smem_u32(dsm) + kRowBytes - 1) & ~(kRowBytes - 1);
+  // planes A and B of W vertices from s0 on, the escape mask, then the per-warp queues of filtered
+  // entry indices
+  uint32_t *deep = reinterpret_cast<uint32_t *>(dsm + (s0 - smem_u32(dsm)) + planes_bytes(g.tile_shift));
+  uint32_t *queue = deep + deep_words(blockDim.x) + warp * kQueueSlots;
+  const uint32_t C = g.C, B = g.B, cap = 1u << min(B, kDepthEscape);
+  for (uint32_t q = threadIdx.x; q < W; q += blockDim.x) s_row[q] = pair_row(s0 >> 8, q);
+  PlaneItem x;
   x.gsk = reinterpret_cast<uint32_t *>(sketches);
-  x.s_kcol = s_kcol;
-  x.kchk = ph.kchk;
-  const uint32_t stride = g.nbins + 1;
-  const uint32_t C = g.C, B = g.B;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const uint32_t t = atomicAdd(work_counter, 1u);
-      uint32_t total = 0;
-      if (t < g.ntiles) {
-        const uint32_t bin = t >> per_bin;
-        for (int k = 0; k < nchunks; ++k)
-          total += bin_off[(uint64_t)k * stride + bin + 1] - bin_off[(uint64_t)k * stride + bin];
-      }
-      s_claim[0] = t;
-      s_claim[1] = total;
+  x.row_of = s_row;
+  x.deep = deep;
+  const uint32_t stride = g.nbins + 1, nitems = g.ntiles * g.groups;
+  for (uint32_t i = threadIdx.x; i < planes_bytes(g.tile_shift) / 16; i += blockDim.x)
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(s0 + i * 16), "r"(0u));
+  auto claim = [&](uint32_t *to) {
+    const uint32_t it = atomicAdd(work_counter, 1u);
+    uint32_t total = 0;
+    if (it < nitems) {
+      const uint32_t bin = (it / g.groups) >> per_bin;
+      for (int k = 0; k < nchunks; ++k)
+        total += bin_off[(uint64_t)k * stride + bin + 1] - bin_off[(uint64_t)k * stride + bin];
     }
+    to[0] = it;
+    to[1] = total;  // entries of the tile's bin
+  };
+  if (threadIdx.x == 0) claim(s_claim[0]);
+  for (uint32_t n = 0;; ++n) {
     __syncthreads();
-    const uint32_t t = s_claim[0], total = s_claim[1];  // total: entries of the tile's bin
-    if (t >= g.ntiles) break;
-    const uint32_t bin = t >> per_bin;
-    if (total == 0) {
-      __syncthreads();
-      continue;
-    }
-    if (total < (g.direct_max << per_bin)) {
-      // few entries: updated in place in HBM (no planes to clear and write back)
-      for (int k = 0; k < nchunks; ++k) {
-        const uint32_t b = bin_off[(uint64_t)k * stride + bin], e = bin_off[(uint64_t)k * stride + bin + 1];
-        const uint8_t *cb = gutter + chunks.base[k];
-        const uint32_t kind = chunks.kind[k];
-        for (uint32_t i = b + threadIdx.x; i < e; i += blockDim.x)
-          entry_in_place(load_entry(cb, kind, i), kind, bin, t, g.tile_shift, x);
-      }
-      __syncthreads();
-      continue;
-    }
-    {
-      uint4 *pz = reinterpret_cast<uint4 *>(planes);
-      const uint32_t n16 = W * (kVertBytes / 16);
-      for (uint32_t i = threadIdx.x; i < n16; i += blockDim.x) pz[i] = make_uint4(0, 0, 0, 0);
-    }
-    __syncthreads();
-    // an invalid lane carries an entry of vertex 0 of the tile with neighbour 0 and no codes
-    const uint4 pad_entry = make_uint4(t << g.tile_shift, 0, 0, 0);
+    const uint32_t item = s_claim[n & 1][0], total = s_claim[n & 1][1];
+    if (item >= nitems) break;
+    if (threadIdx.x == 0) claim(s_claim[(n + 1) & 1]);  // while the others work on this one
+    if (total == 0) continue;
+    const uint32_t grp = g.groups == 1 ? 0u : item % g.groups;
+    x.t = g.groups == 1 ? item : item / g.groups;
+    x.bin = x.t >> per_bin;
+    x.c0 = grp * kPlaneSlots;
+    x.nc = min(C - x.c0, kPlaneSlots);
+    x.kcol = ph.kcol + x.c0;
+    const bool direct = !CUBE && total < (g.direct_max << per_bin);
+    if (direct && grp) continue;
     for (int k = 0; k < nchunks; ++k) {
-      const uint32_t b = bin_off[(uint64_t)k * stride + bin], e = bin_off[(uint64_t)k * stride + bin + 1];
+      const uint32_t b = bin_off[(uint64_t)k * stride + x.bin], e = bin_off[(uint64_t)k * stride + x.bin + 1];
       const uint8_t *cb = gutter + chunks.base[k];
-      const uint32_t kind = chunks.kind[k];
-      // each warp takes groups of 32 entries; the next group is loaded while this one is used
-      uint32_t i0 = b + warp * 32;
-      bool nvalid = i0 + lane < e;
-      uint4 nx = nvalid ? load_entry(cb, kind, i0 + lane) : pad_entry;
-      if (per_bin == 0) {
-        // the bin is this tile: every entry applies
-        for (; i0 < e; i0 += nwarps * 32) {
-          const uint4 en = nx;
-          const bool valid = nvalid;
-          const uint32_t in = i0 + nwarps * 32 + lane;
-          nvalid = in < e;
-          if (nvalid) nx = load_entry(cb, kind, in);
-          plane_entry(en, kind, valid, bin, lane, x);
-        }
-      } else {
-        // the bin holds several tiles: each warp ballots its group, queues this tile's entries,
-        // and applies full warps of queued entries; two groups are in flight ahead of the one
-        // ballotted
-        uint32_t qn = 0;
-        const uint32_t step = nwarps * 32;
-        bool nvalid2 = i0 + step + lane < e;
-        uint4 nx2 = nvalid2 ? load_entry(cb, kind, i0 + step + lane) : pad_entry;
-        for (; i0 < e; i0 += step) {
-          const uint4 en = nx;
-          const bool mine = nvalid && (entry_vertex(en, kind, bin, x) >> g.tile_shift) == t;
-          nx = nx2;
-          nvalid = nvalid2;
-          const uint32_t in = i0 + 2 * step + lane;
-          nvalid2 = in < e;
-          if (nvalid2) nx2 = load_entry(cb, kind, in);
-          const uint32_t m = __ballot_sync(kFull, mine);
-          if (mine) queue[qn + __popc(m & ((1u << lane) - 1u))] = en;
-          qn += __popc(m);
-          __syncwarp();
-          if (qn >= 32) {
-            const uint4 q = queue[lane];
-            __syncwarp();
-            qn -= 32;
-            if (lane < qn) queue[lane] = queue[32 + lane];
-            __syncwarp();
-            plane_entry(q, kind, true, bin, lane, x);
+      const uint32_t kind = CODED ? chunks.kind[k] : kEntryPlain;
+      if (direct) {
+        // few entries: each XORed in place in HBM by a warp, lane by column (no planes to write back)
+        for (uint32_t i = b + warp; i < e; i += nwarps) {
+          uint4 en;
+          uint32_t v, u, w4[4];
+          if (CODED && kind != kEntryPlain) {
+            en = load_entry<kEntryCoded>(cb, i);
+            if (kind == kEntryCoded) unpack_entry(en, x.bin, C, g.bin_shift, v, u, w4);
+            else unpack_entry3(en, x.bin, C, g.bin_shift, v, u, w4);
+          } else {
+            en = load_entry<kEntryPlain>(cb, i);
+            v = en.x;
+            u = en.y;
           }
+          if ((v >> g.tile_shift) != x.t) continue;
+          const uint32_t lo = max(u, v), hi = min(u, v);
+          const uint64_t pm = xxh3_premix(((uint64_t)lo << 32) | hi);
+          warp_update_global(x.gsk + (uint64_t)v * g.sketch_words, C,
+                             depth_exact(pm ^ x.kcol[min(lane, C - 1)], B), B, lo, hi, tail_lo32(pm ^ ph.kchk));
         }
-        const bool valid = lane < qn;
-        const uint4 q = valid ? queue[lane] : pad_entry;
-        __syncwarp();
-        if (qn) plane_entry(q, kind, valid, bin, lane, x);
+        continue;
+      }
+      const uint32_t seg = 32 * deep_words(blockDim.x);
+      for (uint32_t b1 = b; b1 < e; b1 += seg) {
+        const uint32_t e1 = min(e, b1 + seg);
+        if (CODED && kind == kEntryCoded) plane_chunk<kEntryCoded, CUBE>(x, g, ph.kchk, cap, cb, b1, e1, queue);
+        else if (CODED && kind == kEntryCoded3) plane_chunk<kEntryCoded3, CUBE>(x, g, ph.kchk, cap, cb, b1, e1, queue);
+        else plane_chunk<kEntryPlain, CUBE>(x, g, ph.kchk, cap, cb, b1, e1, queue);
       }
     }
-    __syncthreads();
-    // write-back: one warp per vertex. The words of rows 0 .. R - 1 of every column (one run of
-    // 3R words per column in the sketch) are taken as one list: word i of the list is column
-    // i / 3R, row (i % 3R) / 3, word (i % 3R) % 3 of the bucket, converted from the planes, and
-    // XORed into the sketch in HBM where it is not zero. Lane l takes words l, l + 32, ... (runs of
-    // consecutive words: coalesced), eight read-modify-writes in flight at a time.
-    const uint32_t R = min(B, kPlaneThr);
-    const uint32_t runw = 3 * R, nwl = C * runw;
+    if (direct) continue;
+    // the first lines of what the write-back reads are brought to L2 while the other warps finish
     for (uint32_t vl = warp; vl < W; vl += nwarps) {
-      const uint32_t vg = (t << g.tile_shift) + vl;
-      if (vg >= g.V) continue;
-      const uint32_t *pa = reinterpret_cast<const uint32_t *>(planes + (size_t)vl * kVertBytes);
-      const uint32_t *pga = pa + kPlaneRows * kPlaneSlots;
-      const uint32_t *pb = pga + kPlaneRows * kPlaneSlots;
-      const uint32_t *pgb = pb + kPlaneRows * kPlaneSlots;
-      uint32_t *sk = x.gsk + (uint64_t)vg * g.sketch_words;
-      // word (c, w) of lane l's current list position; w < runw
-      uint32_t c = 0, w = lane;
-      while (w >= runw) {
-        w -= runw;
-        ++c;
-      }
-      auto word = [&](uint32_t cc, uint32_t ww) -> uint32_t {
-        const uint32_t r = (ww * 0xAAABu) >> 17;  // ww / 3 for ww < 2^15
-        const uint32_t s = r * kPlaneSlots + cc, kk = ww - 3 * r;
-        const uint32_t a = pa[s], bq = pb[s];
-        return kk == 0 ? (a & 0x7fffffffu) ^ ((bq >> 31) ? vg : 0u)
-             : kk == 1 ? (bq & 0x7fffffffu) ^ ((a >> 31) ? vg : 0u) : pga[s] ^ pgb[s];
-      };
-      for (uint32_t i0 = 0; i0 < nwl; i0 += 8 * 32) {
-        uint32_t y[8], old[8], off[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const bool in = i0 + k * 32 + lane < nwl;
-          y[k] = in ? word(c, w) : 0u;
-          off[k] = 3 * c * B + w;
-          old[k] = y[k] ? sk[off[k]] : 0u;
-          w += 32;
-          while (w >= runw) {
-            w -= runw;
-            ++c;
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (y[k]) sk[off[k]] = old[k] ^ y[k];
-      }
-      if (lane < 3) {  // deterministic bucket: slot C, row 0
-        const uint32_t a = pa[C], bq = pb[C];
-        const uint32_t y = lane == 0 ? (a & 0x7fffffffu) ^ ((bq >> 31) ? vg : 0u)
-                         : lane == 1 ? (bq & 0x7fffffffu) ^ ((a >> 31) ? vg : 0u) : pga[C] ^ pgb[C];
-        if (y) sk[3 * C * B + lane] ^= y;
+      const uint32_t vg = (x.t << g.tile_shift) + vl;
+      if (vg < g.V && lane < x.nc) {
+        const uint32_t *p = x.gsk + (uint64_t)vg * g.sketch_words + 3 * (x.c0 + lane) * B;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+        if (total >= 64u << g.tile_shift) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 3 * min(B, kPlaneThr) - 1));
       }
     }
     __syncthreads();
+    for (uint32_t vl = warp; vl < W; vl += nwarps) {
+      const uint32_t vg = (x.t << g.tile_shift) + vl;
+      if (vg >= g.V) break;
+      write_back<CUBE>(s_row[vl] << 8, vg, x.gsk + (uint64_t)vg * g.sketch_words + 3 * (size_t)x.c0 * B, x.nc,
+                       C - x.c0, B, lane);
+    }
   }
 }
 
@@ -713,16 +893,16 @@ __global__ void k_plane_hash_peak(uint32_t iters, uint64_t *out) {
 }
 
 // Rate of the plane update's shared-memory step alone: 32 vertices of planes, each thread one
-// synthetic entry per iteration (codes 0..3, random vertex and plane), 32 slot steps of two
-// red.shared.xor each, addressed exactly as plane_entry does.
+// synthetic entry per iteration (codes 0..3, random vertex and plane), its 32 slot steps made
+// exactly as the update makes them.
 __global__ void __launch_bounds__(1024, 1) k_plane_update_peak(uint32_t iters, uint32_t *out) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  const uint32_t s0 = smem_u32(dsm);
-  const uint32_t pad = (128u - (s0 & 127u)) & 127u;
-  uint8_t *planes = dsm + pad;
-  const uint32_t sp = s0 + pad, lane = threadIdx.x & 31;
-  uint32_t *pw = reinterpret_cast<uint32_t *>(planes);
-  for (uint32_t i = threadIdx.x; i < kPlaneMaxTile * kVertBytes / 4; i += blockDim.x) pw[i] = 0;
+  __shared__ uint32_t s_row[kPlaneMaxTile];
+  const uint32_t s0 = (smem_u32(dsm) + kRowBytes - 1) & ~(kRowBytes - 1);
+  const uint32_t lane = threadIdx.x & 31, words = planes_bytes(5) / 4;
+  uint32_t *pw = reinterpret_cast<uint32_t *>(dsm + (s0 - smem_u32(dsm)));
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) pw[i] = 0;
+  if (threadIdx.x < kPlaneMaxTile) s_row[threadIdx.x] = pair_row(s0 >> 8, threadIdx.x);
   __syncthreads();
   uint32_t z = fmix32_(blockIdx.x * 1024u + threadIdx.x);
   for (uint32_t it = 0; it < iters; ++it) {
@@ -730,27 +910,11 @@ __global__ void __launch_bounds__(1024, 1) k_plane_update_peak(uint32_t iters, u
     uint32_t c4[4];
 #pragma unroll
     for (int w = 0; w < 4; ++w) c4[w] = fmix32_(z + (uint32_t)w) & 0x33333333u;
-    const uint32_t v = z >> 27, p = (z >> 26) & 1u;
-    const uint32_t val = z | 0x80000000u, chk = z * 747796405u;
-    uint32_t ev[4], od[4];
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      ev[w] = (c4[w] & 0x0f0f0f0fu) << 3;
-      od[w] = ((c4[w] >> 4) & 0x0f0f0f0fu) << 3;
-    }
-    const uint32_t base = sp + v * kVertBytes + p * 2 * kPlaneBytes + (lane << 2);
-#pragma unroll
-    for (int t = 0; t < 32; ++t) {
-      const uint32_t w = (uint32_t)t >> 3, k = ((uint32_t)t & 7u) >> 1;
-      const uint32_t d8 = __byte_perm((t & 1) ? od[w] : ev[w], 0, 0x4440u + k);
-      const uint32_t a = (base + d8 * 16u) ^ (uint32_t)(t << 2);
-      red_xor_shared(a, val);
-      red_xor_shared_g(a, chk);
-    }
+    slot_steps(c4, s_row[z >> 27] + ((z >> 26) & 1u) * kPlaneRows, z | 0x80000000u, z * 747796405u, lane);
   }
   __syncthreads();
   uint32_t acc = 0;
-  for (uint32_t i = threadIdx.x; i < kPlaneMaxTile * kVertBytes / 4; i += blockDim.x) acc ^= pw[i];
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) acc ^= pw[i];
   out[blockIdx.x * 1024u + threadIdx.x] = acc;
 }
 
@@ -772,13 +936,17 @@ PlaneHash plane_hash(uint64_t seed, uint32_t C, uint32_t B) {
 constexpr int kHashSortMaxRpt = 6;
 constexpr int kHashSortThreads = 1024;  // one CTA per SM (every register of the SM)
 
-uint32_t hash_sort_tile(uint32_t nbins, size_t smem_budget) {
+uint32_t hash_sort_tile(uint32_t nbins, size_t smem_budget, uint64_t n) {
   const int nt = kHashSortThreads;
   const size_t fixed = (size_t)2 * ((nbins + 3) & ~3u) * 4 + 256;
   if (nbins > kSortBinsMax || fixed >= smem_budget) return 0;
   // 2 coded entries of 16 B per record, and their 2-byte bins
-  const size_t t = std::min<size_t>((smem_budget - fixed) / 36, (size_t)kHashSortMaxRpt * nt);
-  return (uint32_t)(t / nt * nt);
+  const uint64_t most = std::min<size_t>((smem_budget - fixed) / 36, (size_t)kHashSortMaxRpt * nt) / nt * nt;
+  if (!most) return 0;
+  // an SM's share of the records in as few tiles as hold it, all alike: a short call then uses every
+  // SM (8,528 records: 22 us in two tiles of 6144, 9 us in nine of 1024), a long one has no short last wave
+  const uint64_t share = (n + num_sms() - 1) / num_sms(), k = std::max<uint64_t>(1, (share + most - 1) / most);
+  return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(nt, ((share + k - 1) / k + nt - 1) / nt * nt));
 }
 
 cudaError_t gutter_hash_sort(const void *d_rec, uint64_t n, GutterGeom g, const PlaneHash &ph,
@@ -815,13 +983,14 @@ cudaError_t gutter_hash_sort(const void *d_rec, uint64_t n, GutterGeom g, const 
 }
 
 size_t plane_update_smem(uint32_t tile_shift, int threads) {
-  return 128 + ((size_t)kVertBytes << tile_shift) + (size_t)(threads / 32) * kWbWords * 4;
+  return kRowBytes + planes_bytes(tile_shift) + deep_words(threads) * 4 + (size_t)(threads / 32) * kQueueSlots * 4;
 }
 
 int plane_update_ctas_per_sm(uint32_t tile_shift, int threads) {
   int n = 0;
-  if (smem_optin(k_plane_update) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_plane_update, threads,
+  auto kern = k_plane_update<true, false, PlaneHash>;
+  if (smem_optin(kern) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads,
                                                     plane_update_smem(tile_shift, threads)) != cudaSuccess)
     return 1;
   return n > 0 ? n : 1;
@@ -831,13 +1000,60 @@ cudaError_t plane_update(const PlaneGeom &g, const PlaneHash &ph, uint8_t *sketc
                          const uint8_t *gutter, const ChunkTable &chunks, const uint32_t *bin_off,
                          int nchunks, uint32_t *work_counter, uint32_t * /*status*/, int grid,
                          int threads, cudaStream_t s) {
-  if (g.C > kPlaneMaxColumns || g.C < 18 || g.tile_shift > 5 ||
+  if (g.C > kPlaneMaxColumns || g.C < 18 || g.groups != 1 || g.tile_shift > 5 ||
       g.bin_shift < g.tile_shift || threads % 32 || threads < 32 || threads > 1024)
     return cudaErrorInvalidValue;
-  cudaError_t e = smem_optin(k_plane_update);
+  auto kern = k_plane_update<true, false, PlaneHash>;
+  cudaError_t e = smem_optin(kern);
   if (e != cudaSuccess) return e;
-  k_plane_update<<<grid, threads, plane_update_smem(g.tile_shift, threads), s>>>(
-      g, ph, sketches, gutter, chunks, bin_off, nchunks, work_counter);
+  kern<<<grid, threads, plane_update_smem(g.tile_shift, threads), s>>>(g, ph, sketches, gutter, chunks, bin_off,
+                                                                      nchunks, work_counter);
+  add_launches(1);
+  return cudaGetLastError();
+}
+
+// 32 threads a vertex: one warp each in the write-back. Four CTAs of 8 vertices share an SM, two of 16.
+int plane_threads(uint32_t tile_shift) { return std::min(1024, 32 << tile_shift); }
+
+PlaneHashWide plane_hash_wide(uint64_t seed, uint32_t C, uint32_t B) {
+  PlaneHashWide ph{};
+  ph.C = C;
+  ph.B = B;
+  for (uint32_t c = 0; c < C && c < kPlaneMaxColumnsWide; ++c) ph.kcol[c] = xxh3_premix(xxh3_flip(seed + 5ull * c));
+  ph.kchk = xxh3_premix(xxh3_flip(seed));
+  return ph;
+}
+
+cudaError_t plane_update_plain(const PlaneGeom &g, bool cube, const PlaneHashWide &ph, uint8_t *sketches,
+                               const uint8_t *gutter, const ChunkTable &chunks, const uint32_t *bin_off,
+                               int nchunks, uint32_t *work_counter, cudaStream_t s) {
+  if (g.C > kPlaneMaxColumnsWide || g.groups != (g.C + kPlaneSlots) / kPlaneSlots || g.tile_shift > 5 ||
+      g.bin_shift < g.tile_shift || (g.groups > 1 && g.direct_max))
+    return cudaErrorInvalidValue;
+  const int threads = plane_threads(g.tile_shift);
+  const size_t smem = plane_update_smem(g.tile_shift, threads);
+  auto launch = [&](auto kern) -> cudaError_t {
+    cudaError_t e = smem_optin(kern);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    if (e != cudaSuccess) return e;
+    const int grid = (int)std::min<uint64_t>((uint64_t)g.ntiles * g.groups, (uint64_t)num_sms() * std::max(per_sm, 1));
+    kern<<<grid, threads, smem, s>>>(g, ph, sketches, gutter, chunks, bin_off, nchunks, work_counter);
+    add_launches(1);
+    return cudaGetLastError();
+  };
+  return cube ? launch(k_plane_update<false, true, PlaneHashWide>)
+              : launch(k_plane_update<false, false, PlaneHashWide>);
+}
+
+cudaError_t direct_records(const void *d_rec, uint64_t n, uint32_t V, uint32_t sketch_words,
+                           const PlaneHash &ph, uint8_t *sketches, uint32_t *status, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  if (ph.C > kPlaneMaxColumns) return cudaErrorInvalidValue;
+  const unsigned grid = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)num_sms() * 8);
+  k_direct_records<<<grid, 256, 0, s>>>(reinterpret_cast<const uint8_t *>(d_rec), n, V, sketch_words, ph,
+                                        reinterpret_cast<uint32_t *>(sketches), status);
   add_launches(1);
   return cudaGetLastError();
 }
@@ -851,7 +1067,7 @@ cudaError_t plane_hash_peak(uint32_t iters, int blocks, int threads, uint64_t *o
 cudaError_t plane_update_peak(uint32_t iters, int blocks, uint32_t *out, cudaStream_t s) {
   cudaError_t e = smem_optin(k_plane_update_peak);
   if (e != cudaSuccess) return e;
-  k_plane_update_peak<<<blocks, 1024, 128 + kPlaneMaxTile * kVertBytes, s>>>(iters, out);
+  k_plane_update_peak<<<blocks, 1024, kRowBytes + planes_bytes(5), s>>>(iters, out);
   add_launches(1);
   return cudaGetLastError();
 }
