@@ -25,6 +25,7 @@
 #include "gz_common.cuh"
 #include "gz_device.cuh"
 #include "gz_kernels.cuh"
+#include "gz_planes.cuh"
 
 void gz_internal_set_error(const std::string &msg);
 
@@ -42,7 +43,8 @@ struct GraphDesc {
   uint32_t tile_base; // first global tile
   uint32_t flip_off;  // first of the graph's C + 1 hash constants
   uint32_t nbins, ntiles;
-  uint32_t direct_max;  // tiles with fewer entries are updated in place in HBM, unstaged
+  uint32_t direct_max;  // staged form: tiles with fewer entries are updated in place in HBM
+  uint32_t plane;       // its tiles are those of the bucket-plane form
 };
 
 // ---- gutter ----------------------------------------------------------------------------------
@@ -158,6 +160,91 @@ k_mb_sort_scatter(const uint8_t *__restrict__ rec, const uint4 *__restrict__ rti
   }
 }
 
+// The same with coded entries (gz_planes.cu: each record hashed once, its columns' depth codes carried
+// by both endpoints' entries), the form of calls whose graphs' codes all fit 16 bytes: a hash costs
+// more than the 8 bytes it adds to an entry (128 graphs, 1.17e8 records: sort and update 12.7 -> 9.6 ms).
+constexpr int kMbHashRpt = kMbRecTile / 1024;
+__global__ void __launch_bounds__(1024, 1)
+k_mb_hash_sort(const uint8_t *__restrict__ rec, const uint4 *__restrict__ rtiles, uint32_t n_rt,
+               const GraphDesc *__restrict__ graphs, const uint64_t *__restrict__ flip,
+               const uint64_t *__restrict__ base, uint32_t *__restrict__ fill, uint4 *__restrict__ entries) {
+  extern __shared__ __align__(128) uint8_t bsm128[];
+  __shared__ uint32_t ws[32];
+  __shared__ uint64_t s_kcol[kPlaneSlots];
+  uint32_t *s_cur = reinterpret_cast<uint32_t *>(bsm128);  // counts, then placement cursors
+  uint32_t *s_rel = s_cur + kMbBinsMax;  // a bin's run: gutter position minus position in the tile
+  uint4 *s_ent = reinterpret_cast<uint4 *>(s_rel + kMbBinsMax);
+  uint16_t *s_bin = reinterpret_cast<uint16_t *>(s_ent + 2 * kMbRecTile);
+  uint8_t *s_rec = reinterpret_cast<uint8_t *>(s_ent);  // staged records, parsed before the first entry is placed
+  for (uint32_t t = blockIdx.x; t < n_rt; t += gridDim.x) {
+    const uint4 rt = rtiles[t];
+    const GraphDesc gd = graphs[rt.x];
+    const uint32_t nb = gd.nbins, cnt = rt.w, cap = 1u << min(gd.B, kDepthEscape);
+    const uint32_t per_thread = (nb + blockDim.x - 1) / blockDim.x;  // <= 4
+    if (threadIdx.x < kPlaneSlots)
+      s_kcol[threadIdx.x] = threadIdx.x < gd.C ? xxh3_premix(flip[gd.flip_off + threadIdx.x]) : 0;
+    for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_cur[b] = 0u;
+    const uint32_t shift = stage_records(rec, ((uint64_t)rt.z << 32) | rt.y, cnt, s_rec);
+    __syncthreads();
+    uint32_t ru[kMbHashRpt], rv[kMbHashRpt];
+#pragma unroll
+    for (int k = 0; k < kMbHashRpt; ++k) {
+      const uint32_t i = threadIdx.x + k * blockDim.x;
+      ru[k] = rv[k] = 0xffffffffu;
+      if (i < cnt) {
+        parse_record(s_rec, shift, i, ru[k], rv[k]);
+        if (ru[k] >= gd.V || rv[k] >= gd.V) ru[k] = 0xffffffffu;  // dropped (the count pass flags it)
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kMbHashRpt; ++k)
+      if (ru[k] != 0xffffffffu) {
+        atomicAdd(&s_cur[ru[k] >> gd.bin_shift], 1u);
+        atomicAdd(&s_cur[rv[k] >> gd.bin_shift], 1u);
+      }
+    __syncthreads();
+    uint32_t sum = 0;
+    for (uint32_t k = 0; k < per_thread; ++k) {
+      const uint32_t b = threadIdx.x * per_thread + k;
+      sum += b < nb ? s_cur[b] : 0u;
+    }
+    uint32_t run = block_scan_1024(sum, ws);
+    for (uint32_t k = 0; k < per_thread; ++k) {
+      const uint32_t b = threadIdx.x * per_thread + k;
+      if (b < nb) {
+        const uint32_t c = s_cur[b], gb = gd.bin_base + b;
+        s_rel[b] = c ? (uint32_t)base[gb] + atomicAdd(&fill[gb], c) - run : 0u;
+        s_cur[b] = run;
+        run += c;
+      }
+    }
+    __syncthreads();
+    uint32_t pu[kMbHashRpt], pv[kMbHashRpt];
+#pragma unroll
+    for (int k = 0; k < kMbHashRpt; ++k)
+      if (ru[k] != 0xffffffffu) {
+        pu[k] = atomicAdd(&s_cur[ru[k] >> gd.bin_shift], 1u);
+        pv[k] = atomicAdd(&s_cur[rv[k] >> gd.bin_shift], 1u);
+      }
+#pragma unroll
+    for (int k = 0; k < kMbHashRpt; ++k)
+      if (ru[k] != 0xffffffffu) {
+        const uint64_t pm = xxh3_premix(((uint64_t)max(ru[k], rv[k]) << 32) | min(ru[k], rv[k]));
+        uint32_t w[4];
+        all_codes<18>(pm, s_kcol, gd.C, cap, w);
+        s_ent[pu[k]] = pack_entry(w, ru[k], rv[k], gd.C, gd.bin_shift);
+        s_ent[pv[k]] = pack_entry(w, rv[k], ru[k], gd.C, gd.bin_shift);
+        s_bin[pu[k]] = (uint16_t)(ru[k] >> gd.bin_shift);
+        s_bin[pv[k]] = (uint16_t)(rv[k] >> gd.bin_shift);
+      }
+    __syncthreads();
+    const uint32_t total = s_cur[nb - 1];
+    for (uint32_t j = threadIdx.x; j < total; j += blockDim.x) entries[s_rel[s_bin[j]] + j] = s_ent[j];
+    __syncthreads();
+  }
+}
+constexpr size_t kMbHashSmem = 2 * kMbBinsMax * 4 + (size_t)kMbRecTile * 36;
+
 constexpr size_t kMbCountSmem = kMbBinsMax * 4 + kMbRecTile * 9 + 48;
 constexpr size_t kMbSortSmem = 3 * kMbBinsMax * 4 + 2 * kMbRecTile * 8 + kMbRecTile * 9 + 48;
 
@@ -169,14 +256,44 @@ __global__ void k_mb_bin_off(const uint64_t *scanned, uint64_t nbins, const uint
 }
 
 // ---- sparse route: records applied in place ---------------------------------------------------
-// For a graph whose call brings too few records to pay for the gutter and tile staging, each
-// record is hashed once (checksum and C depths, shared by both endpoints) and XORed into both
-// endpoints' sketches in HBM with global atomics. A self-loop XORs one sketch twice: no change,
-// as in the gutter path.
+// For a graph whose call brings too few records to pay for the gutter and its tiles, each record is
+// hashed once by a warp, a lane per column, and XORed into both endpoints' sketches in HBM with
+// global reductions (warp_record_global: bound by L2's rate for them, about 45e9 sectors/s). A
+// self-loop XORs one sketch twice: no change, as in the gutter path. The warps of the grid take runs
+// of 32 records of the record tiles (32 lanes read them at once). (Sketches of more than 31 columns,
+// k_mb_direct_wide: a thread per record.)
+__global__ void __launch_bounds__(256)
+k_mb_direct(const uint8_t *__restrict__ rec, uint64_t n_rec, const uint4 *__restrict__ rtiles, uint32_t n_rt,
+            const GraphDesc *__restrict__ graphs, uint8_t *__restrict__ sketches,
+            const uint64_t *__restrict__ flip, uint32_t *__restrict__ status) {
+  constexpr uint32_t kRuns = kMbRecTile / 32;
+  const uint32_t lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rt * kRuns; r += nwarps) {
+    const uint4 rt = rtiles[r / kRuns];
+    const uint32_t i0 = (r % kRuns) * 32;
+    if (i0 >= rt.w) continue;
+    const GraphDesc gd = graphs[rt.x];
+    const uint64_t kc = xxh3_premix(flip[gd.flip_off + min(lane, gd.C)]);
+    const uint64_t kchk = xxh3_premix(flip[gd.flip_off + gd.C]);
+    uint32_t *gsk = reinterpret_cast<uint32_t *>(sketches + gd.sk_off);
+    uint32_t mu = 0, mv = 0;
+    if (i0 + lane < rt.w) load_record(rec, rec + 9 * n_rec, (((uint64_t)rt.z << 32) | rt.y) + i0 + lane, mu, mv);
+    if (mu >= gd.V || mv >= gd.V) {
+      atomicOr(status, kStatusBadVertex);
+      mu = mv;  // dropped
+    }
+    for (uint32_t m = __ballot_sync(kFull, mu != mv); m; m &= m - 1) {
+      const uint32_t u = __shfl_sync(kFull, mu, __ffs(m) - 1), v = __shfl_sync(kFull, mv, __ffs(m) - 1);
+      warp_record_global(gsk + (uint64_t)u * gd.sketch_words, gsk + (uint64_t)v * gd.sketch_words, u, v, gd.C, gd.B,
+                         kc, kchk);
+    }
+  }
+}
+
 constexpr uint32_t kMbFlipMax = 64;
 
 __global__ void __launch_bounds__(512)
-k_mb_direct(const uint8_t *__restrict__ rec, const uint4 *__restrict__ rtiles, uint32_t n_rt,
+k_mb_direct_wide(const uint8_t *__restrict__ rec, const uint4 *__restrict__ rtiles, uint32_t n_rt,
             const GraphDesc *__restrict__ graphs, uint8_t *__restrict__ sketches,
             const uint64_t *__restrict__ flip, uint32_t *__restrict__ status) {
   extern __shared__ __align__(128) uint8_t dsm[];
@@ -223,16 +340,16 @@ k_mb_direct(const uint8_t *__restrict__ rec, const uint4 *__restrict__ rtiles, u
 
 constexpr size_t kMbDirectSmem = kMbFlipMax * 8 + kMbRecTile * 9 + 48;
 
-// Work list of the tile kernel: the global tiles whose gutter bin holds entries.
+// Work list of a tile kernel: the global tiles of its form (plane) whose gutter bin holds entries.
 __global__ void k_mb_worklist(const GraphDesc *__restrict__ graphs, const uint32_t *__restrict__ tile_graph,
-                              uint32_t total_tiles, const uint32_t *__restrict__ bin_off,
+                              uint32_t total_tiles, const uint32_t *__restrict__ bin_off, uint32_t plane,
                               uint32_t *__restrict__ list, uint32_t *__restrict__ count) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   bool take = false;
   if (t < total_tiles) {
     const GraphDesc gd = graphs[tile_graph[t]];
     const uint32_t bin = gd.bin_base + ((t - gd.tile_base) >> (gd.bin_shift - gd.tile_shift));
-    take = bin_off[bin + 1] > bin_off[bin];
+    take = gd.plane == plane && bin_off[bin + 1] > bin_off[bin];
   }
   const uint32_t m = __ballot_sync(kFull, take);
   uint32_t base = 0;
@@ -434,6 +551,118 @@ k_mb_sketch_update(const GraphDesc *__restrict__ graphs, const uint32_t *__restr
       fence_proxy_async_smem();  // this thread's bucket writes, before the bulk write-back
     }
     mbar_arrive(smem_u32(&s_empty[s]));
+  }
+}
+
+// The default form of the update: tiles of 8 vertices accumulated in bucket planes (gz_planes.cuh), four
+// CTAs of 256 threads per SM whose phases overlap each other. Against the staged tiles above (the
+// form of explicit tile sizes and CTA shapes, and of sketches of more than 31 columns) nothing but
+// the touched words of a sketch moves over HBM, and the bucket updates have no bank conflicts
+// (128 graphs, 1.17e8 records, plain entries: 13.3 -> 10.4 ms).
+struct MbPlaneItem {
+  uint32_t item, lt, b, e;  // work item, tile in its graph, entry range of its bin
+  uint32_t g, V, C, B, words, bin_shift, flip_off, pad;
+  uint64_t sk_off;
+};
+constexpr uint32_t kMbPlaneShift = 3;
+constexpr uint32_t kMbPlaneThreads = 32u << kMbPlaneShift;
+constexpr uint32_t kMbClaim = 4;  // items claimed at once when there are many
+constexpr size_t kMbPlaneSmem = kRowBytes + planes_bytes(kMbPlaneShift) + deep_words(kMbPlaneThreads) * 4 +
+                                kMbPlaneThreads / 32 * kQueueSlots * 4;
+
+// KIND: kEntryPlain or kEntryCoded, of every entry of the launch.
+template <int KIND>
+__global__ void __launch_bounds__(kMbPlaneThreads, 4)
+k_mb_plane_update(const GraphDesc *__restrict__ graphs, const uint32_t *__restrict__ tile_graph,
+                  const uint32_t *__restrict__ worklist, const uint32_t *__restrict__ worklist_len,
+                  uint8_t *__restrict__ sketches, const void *__restrict__ entries,
+                  const uint32_t *__restrict__ bin_off, const uint64_t *__restrict__ flip,
+                  uint32_t *work_counter) {
+  extern __shared__ __align__(128) uint8_t dsm[];
+  __shared__ MbPlaneItem s_item[2 * kMbClaim];
+  __shared__ uint64_t s_kcol[kPlaneSlots];
+  __shared__ uint64_t s_kchk;
+  __shared__ uint32_t s_row[1u << kMbPlaneShift];
+  constexpr uint32_t W = 1u << kMbPlaneShift, nwarps = kMbPlaneThreads / 32;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t s0 = (smem_u32(dsm) + kRowBytes - 1) & ~(kRowBytes - 1);
+  uint32_t *deep = reinterpret_cast<uint32_t *>(dsm + (s0 - smem_u32(dsm)) + planes_bytes(kMbPlaneShift));
+  uint32_t *queue = deep + deep_words(kMbPlaneThreads) + warp * kQueueSlots;
+  const uint32_t nitems = *worklist_len;
+  const uint32_t K = nitems > 16 * kMbClaim * gridDim.x ? kMbClaim : 1u;
+  if (threadIdx.x < W) s_row[threadIdx.x] = pair_row(s0 >> 8, threadIdx.x);
+  for (uint32_t i = threadIdx.x; i < planes_bytes(kMbPlaneShift) / 16; i += blockDim.x)
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(s0 + i * 16), "r"(0u));
+  // the last warp claims the items of iterations n .. n + K - 1, a lane each
+  auto claim = [&](uint32_t n) {
+    uint32_t first = 0;
+    if (lane == 0) first = atomicAdd(work_counter, K);
+    first = __shfl_sync(kFull, first, 0);
+    if (lane >= K) return;
+    MbPlaneItem m{};
+    m.item = first + lane;
+    if (m.item < nitems) {
+      const uint32_t tile = worklist[m.item];
+      m.g = tile_graph[tile];
+      const GraphDesc gd = graphs[m.g];
+      m.lt = tile - gd.tile_base;
+      const uint32_t bin = gd.bin_base + (m.lt >> (gd.bin_shift - gd.tile_shift));
+      m.b = bin_off[bin];
+      m.e = bin_off[bin + 1];
+      m.V = gd.V;
+      m.C = gd.C;
+      m.B = gd.B;
+      m.words = gd.sketch_words;
+      m.bin_shift = gd.bin_shift;
+      m.flip_off = gd.flip_off;
+      m.sk_off = gd.sk_off;
+    }
+    s_item[(n + lane) % (2 * K)] = m;
+  };
+  if (warp == nwarps - 1) claim(0);
+  uint32_t cur_g = 0xffffffffu;
+  for (uint32_t n = 0;; ++n) {
+    __syncthreads();
+    const MbPlaneItem &m = s_item[n % (2 * K)];
+    if (m.item >= nitems) break;
+    if (n % K == 0 && warp == nwarps - 1) claim(n + K);  // while the others work
+    if (m.g != cur_g) {
+      cur_g = m.g;
+      if (threadIdx.x < m.C) s_kcol[threadIdx.x] = xxh3_premix(flip[m.flip_off + threadIdx.x]);
+      else if (threadIdx.x < kPlaneSlots) s_kcol[threadIdx.x] = 0;
+      if (threadIdx.x == 0) s_kchk = xxh3_premix(flip[m.flip_off + m.C]);
+      __syncthreads();
+    }
+    PlaneGeom g;
+    g.B = m.B;
+    g.C = m.C;
+    g.sketch_words = m.words;
+    g.tile_shift = kMbPlaneShift;
+    g.bin_shift = m.bin_shift;
+    PlaneItem x;
+    x.t = m.lt;
+    x.bin = m.lt >> (m.bin_shift - kMbPlaneShift);
+    x.c0 = 0;
+    x.nc = m.C;
+    x.kcol = s_kcol;
+    x.gsk = reinterpret_cast<uint32_t *>(sketches + m.sk_off);
+    x.row_of = s_row;
+    x.deep = deep;
+    const uint32_t cap = 1u << min(m.B, kDepthEscape), total = m.e - m.b, V = m.V;
+    const uint8_t *cb = reinterpret_cast<const uint8_t *>(entries);
+    const uint32_t seg = KIND == kEntryPlain ? 0xffffffffu : 32 * deep_words(kMbPlaneThreads), e = m.e;
+    for (uint32_t b = m.b; b < e; b += min(seg, e - b))
+      plane_chunk<KIND, false>(x, g, s_kchk, cap, cb, b, min(seg, e - b) + b, queue);
+    const uint32_t vl = warp, vg = (x.t << kMbPlaneShift) + vl;  // a warp a vertex
+    uint32_t *sk = x.gsk + (uint64_t)vg * g.sketch_words;
+    if (vg < V && lane < x.nc) {
+      // what the write-back touches first is brought to L2 while the other warps finish
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(sk + 3 * lane * g.B));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(sk + 3 * lane * g.B + 16));
+    }
+    __syncthreads();
+    if (vg < V)
+      write_back<false>(s_row[vl] << 8, vg, sk, x.nc, x.nc, g.B, lane, total < (64u << g.bin_shift));
   }
 }
 
@@ -1200,15 +1429,19 @@ size_t tile_budget(const gz_batch *h, uint32_t max_C) {
 // Tile and bin geometry of one graph. A requested vertices-per-tile (vpt != 0) is used as given;
 // otherwise the largest power of two <= 64 whose tile fits `budget` bytes (a batch has enough
 // tiles to fill the GPU, and bigger tiles spread the shared-memory atomics over more buckets).
-int choose_tiles(GraphDesc &gd, uint32_t vpt, size_t budget) {
+// plane: the bucket-plane form, tiles of 8 vertices whatever the sketches' size.
+int choose_tiles(GraphDesc &gd, uint32_t vpt, size_t budget, bool plane) {
   const uint64_t sketch_bytes = (uint64_t)gd.sketch_words * 4;
   uint32_t shift = 2;
-  if (vpt) {
+  gd.plane = plane ? 1 : 0;
+  if (plane) {
+    shift = kMbPlaneShift;
+  } else if (vpt) {
     shift = (uint32_t)__builtin_ctz(vpt);
   } else {
     while (shift < 6 && (sketch_bytes << (shift + 1)) <= budget) ++shift;
   }
-  if ((sketch_bytes << shift) > budget) return mb_fail(GZ_ERR_INVALID, "sketch too large for a tile");
+  if (!plane && (sketch_bytes << shift) > budget) return mb_fail(GZ_ERR_INVALID, "sketch too large for a tile");
   uint32_t bshift = shift;
   while (((gd.V + (1u << bshift) - 1) >> bshift) > kMbBinTarget && (1u << (bshift - shift)) < 16) ++bshift;
   while (((gd.V + (1u << bshift) - 1) >> bshift) > kMbBinsMax && (1u << (bshift - shift)) < kMbTilesPerBinMax)
@@ -1224,6 +1457,12 @@ int choose_tiles(GraphDesc &gd, uint32_t vpt, size_t budget) {
   // sector read and written per bucket, C + 1 buckets per entry: in place wins below this.
   gd.direct_max = (uint32_t)((sketch_bytes << shift) / (32ull * (gd.C + 1)));
   return GZ_OK;
+}
+
+// Whether a graph can take the bucket-plane form: at most 31 columns, and bins enough for tiles of 8
+// vertices.
+bool plane_fits(const GraphDesc &gd) {
+  return gd.C <= kPlaneMaxColumns && gd.V <= (uint64_t)kMbBinsMax * kMbTilesPerBinMax << kMbPlaneShift;
 }
 
 // Device bytes of one graph's sketches: V rounded up to 64 (any tile stays inside), 256-aligned.
@@ -1265,7 +1504,7 @@ int finalize_graphs(gz_batch *h) {
     tile_base += gd.ntiles;
     h->max_B = std::max(h->max_B, gd.B);
     h->max_C = std::max(h->max_C, gd.C);
-    h->max_tile_bytes = std::max<uint32_t>(h->max_tile_bytes, (gd.sketch_words * 4) << gd.tile_shift);
+    if (!gd.plane) h->max_tile_bytes = std::max<uint32_t>(h->max_tile_bytes, (gd.sketch_words * 4) << gd.tile_shift);
   }
   if (vbase > 0xFFFFFFF0ull || bin_base > 0xFFFFFFF0ull || tile_base > 0xFFFFFFF0ull)
     return mb_fail(GZ_ERR_INVALID, "batch too large for 32-bit global vertex ids");
@@ -1303,7 +1542,10 @@ int layout(gz_batch *h, const std::vector<uint32_t> &vpt_req) {
   uint64_t sk_off = 0, flip_off = 0;
   for (uint32_t g = 0; g < h->graphs.size(); ++g) {
     GraphDesc &gd = h->graphs[g];
-    MB_TRY(choose_tiles(gd, vpt_req.empty() ? 0 : vpt_req[g], budget));
+    const uint32_t vpt = vpt_req.empty() ? 0 : vpt_req[g];
+    // bucket planes unless a tile size or a CTA shape is asked for
+    const bool plane = !vpt && h->threads == 1024 && h->ctas_per_sm == 1 && plane_fits(gd);
+    MB_TRY(choose_tiles(gd, vpt, budget, plane));
     gd.sk_off = sk_off;
     gd.flip_off = (uint32_t)flip_off;
     sk_off += graph_sketch_bytes(gd);
@@ -1327,10 +1569,13 @@ int batch_flush_status(gz_batch *h) {
   return GZ_OK;
 }
 
-// Whether graph gd takes n records of one call in place (sparse route): staging its touched
-// tiles moves about 2 x V x sketch bytes over HBM plus the gutter's bytes, updating in place
-// about 2 (C + 1) bucket sectors of 64 B read + written per record.
+// Whether graph gd takes n records of one call in place (sparse route). Bucket planes: a record in
+// place costs about 2 x 30 sector reductions (1.3 ns of the GPU at L2's 45e9 a second), a tile of 8
+// vertices with few entries about 25 ns: in place while the call brings fewer than about 4 entries a
+// vertex. Staged tiles: staging the touched tiles moves about 2 x V x sketch bytes over HBM plus the
+// gutter's bytes, in place takes about 2 (C + 1) bucket sectors of 64 B per record.
 bool route_sparse(const gz_batch *h, const GraphDesc &gd, uint64_t n) {
+  if (gd.plane) return 2.0 * (double)n < 4.0 * gd.V * h->sparse_factor;
   const double staged = 2.0 * gd.V * (gd.sketch_words * 4.0) + 50.0 * n;
   const double in_place = 128.0 * (gd.C + 1) * (double)n;
   return in_place < staged * h->sparse_factor;
@@ -1366,9 +1611,20 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
   rt_dense.insert(rt_dense.end(), rt_sparse.begin(), rt_sparse.end());
   MB_CUDA(cudaMemcpyAsync(h->d_rtiles, rt_dense.data(), sizeof(uint4) * n_rt, cudaMemcpyHostToDevice, h->stream));
   const uint32_t n_rt_dense = (uint32_t)(n_rt - rt_sparse.size());
+  bool coded = true;
   const uint8_t *rec = static_cast<const uint8_t *>(d_rec);
   if (n_rt_dense) {
-    MB_TRY(grow(&h->d_entries, h->entry_cap, 2 * n_dense, h->stream));
+    // coded entries (16 bytes) when every guttered graph's codes fit them, else plain ones (8)
+    for (uint32_t g = 0; g < h->G && coded; ++g) {
+      const GraphDesc &gd = h->graphs[g];
+      if (off[g + 1] > off[g] && !route_sparse(h, gd, off[g + 1] - off[g]))
+        coded = gd.plane && coded_entry_fits(gd.V, gd.C, gd.bin_shift);
+    }
+    if (coded && grow(&h->d_entries, h->entry_cap, 4 * n_dense, h->stream) != GZ_OK) {
+      cudaGetLastError();
+      coded = false;
+    }
+    if (!coded) MB_TRY(grow(&h->d_entries, h->entry_cap, 2 * n_dense, h->stream));
     MB_TRY(grow(&h->d_worklist, h->cap_worklist, h->total_tiles, h->stream));
     MB_TRY(mb_alloc(&h->d_wl_len, 1));
     MB_CUDA(cudaMemsetAsync(h->d_bins, 0, sizeof(uint64_t) * h->total_bins, h->stream));
@@ -1391,42 +1647,73 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
                                                                        h->d_bin_off);
     h->launches++;
     {
-      MB_CUDA(smem_optin(k_mb_sort_scatter));
       const unsigned grid = (unsigned)std::min<uint64_t>(n_rt_dense, (uint64_t)num_sms());
-      k_mb_sort_scatter<<<grid, 1024, kMbSortSmem, h->stream>>>(rec, h->d_rtiles, n_rt_dense, h->d_graphs,
+      MB_CUDA(smem_optin(k_mb_hash_sort));
+      MB_CUDA(smem_optin(k_mb_sort_scatter));
+      if (coded)
+        k_mb_hash_sort<<<grid, 1024, kMbHashSmem, h->stream>>>(rec, h->d_rtiles, n_rt_dense, h->d_graphs, h->d_flip,
+                                                               h->d_bins, h->d_bin_fill,
+                                                               reinterpret_cast<uint4 *>(h->d_entries));
+      else
+        k_mb_sort_scatter<<<grid, 1024, kMbSortSmem, h->stream>>>(rec, h->d_rtiles, n_rt_dense, h->d_graphs,
                                                                 h->d_bins, h->d_bin_fill, h->d_entries);
       h->launches++;
       MB_CUDA(cudaGetLastError());
     }
-    k_mb_worklist<<<cdiv(h->total_tiles, 256), 256, 0, h->stream>>>(
-        h->d_graphs, h->d_tile_graph, (uint32_t)h->total_tiles, h->d_bin_off, h->d_worklist, h->d_wl_len);
-    h->launches++;
-    MB_CUDA(cudaGetLastError());
   }
   if (h->prof) cudaEventRecord(e1, h->stream);
   if (n_rt_dense) {
-    // one persistent launch over every non-empty tile
-    MB_CUDA(cudaMemsetAsync(h->d_status + 1, 0, sizeof(uint32_t), h->stream));
-    const uint32_t tile_stride = (h->max_tile_bytes + 127) & ~127u;
-    const uint32_t flip_stride = ((h->max_C + 2) & ~1u) * 8;
-    const size_t ksmem = 2 * (size_t)tile_stride + 2 * (size_t)flip_stride + (size_t)(h->threads / 32) * 256;
-    MB_CUDA(smem_optin(k_mb_sketch_update));
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mb_sketch_update, (int)h->threads, ksmem);
-    const int grid = (int)std::min<uint64_t>(h->total_tiles, (uint64_t)num_sms() * std::max(per_sm, 1));
-    k_mb_sketch_update<<<grid, h->threads, ksmem, h->stream>>>(
-        h->d_graphs, h->d_tile_graph, h->d_worklist, h->d_wl_len, h->d_sk, h->d_entries, h->d_bin_off,
-        h->d_flip, tile_stride, flip_stride, h->d_status + 1, h->d_status);
-    h->launches++;
-    MB_CUDA(cudaGetLastError());
+    // one persistent launch over every non-empty tile of each form
+    bool form[2] = {false, false};
+    for (const GraphDesc &gd : h->graphs) form[gd.plane] = true;
+    for (uint32_t plane = 0; plane < 2; ++plane) {
+      if (!form[plane]) continue;
+      MB_CUDA(cudaMemsetAsync(h->d_status + 1, 0, sizeof(uint32_t), h->stream));
+      if (form[0] && plane) MB_CUDA(cudaMemsetAsync(h->d_wl_len, 0, sizeof(uint32_t), h->stream));
+      k_mb_worklist<<<cdiv(h->total_tiles, 256), 256, 0, h->stream>>>(h->d_graphs, h->d_tile_graph,
+                                                                       (uint32_t)h->total_tiles, h->d_bin_off, plane,
+                                                                       h->d_worklist, h->d_wl_len);
+      h->launches++;
+      MB_CUDA(cudaGetLastError());
+      int per_sm = 1;
+      if (plane) {
+        auto kern = coded ? k_mb_plane_update<kEntryCoded> : k_mb_plane_update<kEntryPlain>;
+        MB_CUDA(smem_optin(kern));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)kMbPlaneThreads, kMbPlaneSmem);
+        const int grid = (int)std::min<uint64_t>(h->total_tiles, (uint64_t)num_sms() * std::max(per_sm, 1));
+        kern<<<grid, kMbPlaneThreads, kMbPlaneSmem, h->stream>>>(h->d_graphs, h->d_tile_graph, h->d_worklist,
+                                                                 h->d_wl_len, h->d_sk, h->d_entries, h->d_bin_off,
+                                                                 h->d_flip, h->d_status + 1);
+      } else {
+        const uint32_t tile_stride = (h->max_tile_bytes + 127) & ~127u;
+        const uint32_t flip_stride = ((h->max_C + 2) & ~1u) * 8;
+        const size_t ksmem = 2 * (size_t)tile_stride + 2 * (size_t)flip_stride + (size_t)(h->threads / 32) * 256;
+        MB_CUDA(smem_optin(k_mb_sketch_update));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mb_sketch_update, (int)h->threads, ksmem);
+        const int grid = (int)std::min<uint64_t>(h->total_tiles, (uint64_t)num_sms() * std::max(per_sm, 1));
+        k_mb_sketch_update<<<grid, h->threads, ksmem, h->stream>>>(
+            h->d_graphs, h->d_tile_graph, h->d_worklist, h->d_wl_len, h->d_sk, h->d_entries, h->d_bin_off, h->d_flip,
+            tile_stride, flip_stride, h->d_status + 1, h->d_status);
+      }
+      h->launches++;
+      MB_CUDA(cudaGetLastError());
+    }
   }
   if (!rt_sparse.empty()) {
-    MB_CUDA(smem_optin(k_mb_direct));
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mb_direct, 512, kMbDirectSmem);
-    const unsigned grid = (unsigned)std::min<uint64_t>(rt_sparse.size(), (uint64_t)num_sms() * std::max(per_sm, 1));
-    k_mb_direct<<<grid, 512, kMbDirectSmem, h->stream>>>(rec, h->d_rtiles + n_rt_dense, (uint32_t)rt_sparse.size(),
-                                                         h->d_graphs, h->d_sk, h->d_flip, h->d_status);
+    if (h->max_C <= kPlaneMaxColumns) {
+      const uint64_t warps = rt_sparse.size() * (kMbRecTile / 32);
+      const unsigned grid = (unsigned)std::min<uint64_t>((warps + 7) / 8, (uint64_t)num_sms() * 8);
+      k_mb_direct<<<grid, 256, 0, h->stream>>>(rec, off[h->G], h->d_rtiles + n_rt_dense, (uint32_t)rt_sparse.size(),
+                                               h->d_graphs, h->d_sk, h->d_flip, h->d_status);
+    } else {
+      MB_CUDA(smem_optin(k_mb_direct_wide));
+      int per_sm = 1;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mb_direct_wide, 512, kMbDirectSmem);
+      const unsigned grid = (unsigned)std::min<uint64_t>(rt_sparse.size(), (uint64_t)num_sms() * std::max(per_sm, 1));
+      k_mb_direct_wide<<<grid, 512, kMbDirectSmem, h->stream>>>(rec, h->d_rtiles + n_rt_dense,
+                                                                (uint32_t)rt_sparse.size(), h->d_graphs, h->d_sk,
+                                                                h->d_flip, h->d_status);
+    }
     h->launches++;
     MB_CUDA(cudaGetLastError());
   }
@@ -1935,7 +2222,26 @@ int gz_batch_autotune(gz_batch_t *h, uint32_t records_per_vertex, uint32_t *vpt_
       best_vpt = pick;
     }
   }
+  // the default form (bucket planes where they fit), timed the same way
+  double planes_total = 0;
+  MB_TRY(gz_batch_set_tuning(sc, 0, 0, nullptr));
+  for (uint32_t k = 0; k < K; ++k) {
+    std::vector<uint64_t> o(S + 1);
+    for (uint32_t g = 0; g <= S; ++g) o[g] = std::min(std::max(off[g], off[first[k]]), off[first[k + 1]]);
+    double t = 1e300;
+    for (int rep = 0; rep < 3; ++rep) {
+      gz_batch_set_profiling(sc, 1);
+      MB_TRY(gz_batch_ingest_device(sc, guard.rec, o.data()));
+      if (rep) t = std::min(t, sc->prof_sketch_ms);
+    }
+    planes_total += t;
+  }
   gz_batch_set_profiling(sc, 0);
+  if (planes_total <= best_total) {
+    MB_TRY(gz_batch_set_tuning(h, 0, 0, nullptr));
+    for (uint32_t g = 0; vpt_out && g < h->G; ++g) vpt_out[g] = 1u << h->graphs[g].tile_shift;
+    return GZ_OK;
+  }
   std::vector<uint32_t> vpt(h->G);
   for (uint32_t g = 0; g < h->G; ++g) vpt[g] = best_vpt[cls_of[g]];
   MB_TRY(gz_batch_set_tuning(h, best_shape.threads, best_shape.ctas, vpt.data()));
@@ -2268,7 +2574,7 @@ int gz_server_admit(gz_server_t *s, uint32_t num_vertices, uint64_t seed, uint32
   if (gd.B > 63 || gd.C > kServeTileC) return mb_fail(GZ_ERR_INVALID, "sketch geometry not supported by the server");
   gd.sketch_words = (gd.C * gd.B + 1) * 3;
   const size_t budget = tile_budget(&s->ingest, kServeTileC);
-  MB_TRY(choose_tiles(gd, 0, budget));
+  MB_TRY(choose_tiles(gd, 0, budget, plane_fits(gd)));
   t.bytes = graph_sketch_bytes(gd);
   uint64_t off = 0;
   if (s->used + t.bytes > s->budget || !s->arena_alloc.alloc(t.bytes, off))
