@@ -1,5 +1,5 @@
 // gz_batch.cu -- many independent graph streams on one GPU: one gutter pass and one persistent
-// sketch-update launch for all graphs, and a batched Boruvka whose round is a captured CUDA graph.
+// sketch-update launch for all graphs, and a batched Boruvka in one cooperative launch.
 //
 // Every graph keeps its own sketch geometry (vertex count, seed, columns, buckets per column) and
 // its own shared-memory tile size; a device table describes them. Vertices of all graphs share one
@@ -1143,6 +1143,359 @@ __global__ void k_mb_unite(MBBufs b, int round0) {
   mb_handle(r == kResFail ? 2 : 0, r, g, b.graphs[g], b);
 }
 
+// ---- the whole batched query in one launch -----------------------------------------------------
+// boruvka_emulation of every graph at once, as the single-graph query of gz_query.cu (see there for the
+// form and what bounds it): round 0, then per round an accumulating and a sampling phase, each
+// closed by a barrier of the cooperative launch. lastmod[g] = 1 + the last round that graph g FAILed
+// or merged in; g takes part in round r while lastmod[g] == r and r is below its columns, so its
+// rounds are lastmod[g] in the end, out of samples when they reach its columns. *go = 1 + the last
+// round after which any graph goes on.
+struct MbQuery {
+  uint32_t *rstate, *racc, *det;                     // per vertex: state, accumulator, deterministic bucket
+  uint32_t *lastmod, *ncc, *go, *qbar, *labels;
+  uint32_t sw, G;  // words of an accumulator; graphs
+};
+constexpr int kMbqMaxThreads = 768;
+// the ring's stage (its words + 3) also holds the 32 words of a warp's permutation
+__host__ __device__ inline uint32_t mbq_ring_words(uint32_t acc_words) {
+  return acc_words - 3 > 29u ? acc_words - 3 : 29u;
+}
+
+// sample_batch of gz_query.cu for members of different graphs: lane k holds member k's buckets per
+// column and checksum constant.
+__device__ __forceinline__ int mb_sample_batch(const uint8_t *slots, uint32_t slot_bytes, uint32_t run_cap,
+                                               uint32_t offs, uint32_t B, uint64_t chk, uint32_t n, uint32_t lane0,
+                                               uint64_t *idx) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t k = (lane - lane0) & (kMbKB - 1);
+  const uint32_t ok = __shfl_sync(kFull, offs, k);
+  const bool mine = lane >= lane0 && lane - lane0 < n;
+  const uint8_t *sl = slots + k * slot_bytes;
+  const uint32_t *det = reinterpret_cast<const uint32_t *>(sl + run_cap + (ok >> 8));
+  const bool zero = mine && (det[0] | det[1] | det[2]) == 0;
+  const uint32_t nmax = __reduce_max_sync(kFull, lane < n ? B + 1 : 0u);
+  int first = -1;
+  for (uint32_t q = 0; q < nmax; q += 16) {
+    if (!__any_sync(kFull, mine && !zero && first < 0)) break;
+#pragma unroll
+    for (uint32_t p = 0; p < kMbKB / 2; ++p) {
+      const uint32_t m = min(2 * p + lane / 16, n - 1), pos = q + lane % 16;
+      const uint32_t o = __shfl_sync(kFull, offs, m), nb = __shfl_sync(kFull, B, m) + 1;
+      const uint64_t ck = __shfl_sync(kFull, (unsigned long long)chk, m);
+      const uint32_t at = min(pos, nb - 1);
+      const uint32_t *w = reinterpret_cast<const uint32_t *>(
+          slots + m * slot_bytes + (at ? (o & 255u) + 12 * (at - 1) : run_cap + (o >> 8)));
+      const uint32_t bal = __ballot_sync(kFull, pos < nb && bucket_good(w[0], w[1], w[2], ck));
+      const uint32_t bits = (bal >> (16 * (k & 1))) & 0xffffu;
+      if (k / 2 == p && first < 0 && bits) first = (int)(q + __ffs(bits) - 1);
+    }
+  }
+  *idx = 0;
+  if (!mine || zero) return 1;
+  if (first < 0) return 2;
+  const uint32_t *w = first ? reinterpret_cast<const uint32_t *>(sl + (ok & 255u)) + 3 * (first - 1) : det;
+  *idx = ((uint64_t)w[1] << 32) | w[0];
+  return 0;
+}
+
+// Sets a word that thousands of threads set to the same value: once set, the others only read it,
+// from their SM's L1 (a stale value costs a store). Plain stores queued up at one slice of L2: 6.4 ms for
+// the query of 128 graphs of 1.5e6 vertices, 2.6 with this (3.5 in the grouping rounds, plus 9 host round trips).
+__device__ __forceinline__ void mark(uint32_t *w, uint32_t value) {
+  if (__ldca(w) != value) __stcg(w, value);
+}
+
+// Applies a result of graph g's round: FAIL and merges mark the graph (and the launch when the graph
+// has a next round). The link order is on graph-local ids (see mb_unite).
+__device__ __forceinline__ void mb_apply(int res, uint64_t idx, uint32_t round, uint32_t g, const GraphDesc &gd,
+                                         const MBBufs &b, const MbQuery &q) {
+  if (res == 1) return;
+  if (res == 0) {
+    uint32_t x = (uint32_t)(idx >> 32), y = (uint32_t)idx;
+    if (x >= gd.V || y >= gd.V) {
+      atomicOr(b.status, kStatusBadSample);
+      return;
+    }
+    x += gd.vbase;
+    y += gd.vbase;
+    if (!unite_two(b.parent, x, y, gd.vbase)) return;
+    q.rstate[2 * x + 1] = round + 1;
+  }
+  mark(q.lastmod + g, round + 1);
+  if (round + 1 < gd.C) mark(q.go, round + 1);
+}
+
+// NW: words of a column per lane (4 up to B = 42).
+template <int NW>
+__global__ void __launch_bounds__(kMbqMaxThreads, 1) k_mb_query(MBBufs b, MbQuery q) {
+  constexpr uint32_t BPG = 32 / kMbKB;
+  extern __shared__ __align__(16) uint8_t mb_smem[];
+  const uint32_t V = b.total_V, tid = threadIdx.x, lane = tid & 31, SW = q.sw;
+  const uint32_t ring_words = mbq_ring_words(b.acc_words);
+  BvRing ring;
+  ring.init(mb_smem + (tid >> 5) * bv_warp_bytes(ring_words, kMbKB), ring_words, kMbKB);
+  uint32_t *perm = ring.stage;  // 32 words
+  uint32_t T = 0, nbar = 0;
+  bool failed = false;
+  auto sync = [&]() { return launch_barrier<false>(q.qbar, ++nbar, failed, b.status); };
+  const uint32_t gw = (blockIdx.x * blockDim.x + tid) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t gt = blockIdx.x * blockDim.x + tid, nthreads = gridDim.x * blockDim.x;
+  const uint32_t nbatch = (V + kMbKB - 1) / kMbKB;
+  auto my_vertex = [&](uint32_t it) {
+    const uint32_t bt = it + (lane / kMbKB) * nwarps, v = bt * kMbKB + lane % kMbKB;
+    return bt < nbatch && v < V ? v : 0xffffffffu;
+  };
+  uint32_t r_ahead = 0, g_ahead = 0;  // label and graph of the next vertex of this lane
+  auto ahead = [&](uint32_t it) {
+    const uint32_t v = my_vertex(it);
+    if (v != 0xffffffffu) {
+      r_ahead = __ldcg(b.label + v);
+      g_ahead = b.gov[v];
+    }
+  };
+  auto landed = [&](uint32_t t, bool more) {
+    if (ring.wait(T + t)) return true;
+    if (lane == 0) atomicOr(b.status, kStatusTimeout);
+    if (more) ring.wait(T + t + 1);  // its copies must land before the shared memory is freed
+    failed = true;
+    return false;
+  };
+  for (uint32_t v = gt; v < V; v += nthreads) {
+    b.parent[v] = v;
+    b.label[v] = v;
+    reinterpret_cast<uint2 *>(q.rstate)[v] = make_uint2(0, 0);
+  }
+  for (uint32_t g = gt; g < q.G; g += nthreads) q.lastmod[g] = q.ncc[g] = 0;
+  if (gt == 0) *q.go = 0;
+  if (!sync()) return;
+
+  for (uint32_t it = gw; it < nbatch && !failed; it += BPG * nwarps) {  // round 0
+    const uint32_t v = my_vertex(it);
+    MbVert me{};
+    if (v != 0xffffffffu) me = mb_vert(b, v);
+    uint32_t offs = 0;
+    auto issue = [&](uint32_t t) {  // batch t: the vertices of lanes 8 t .. 8 t + 7
+      const MbVert mk = mb_vert_shfl(me, (t * kMbKB + lane) & 31);
+      const uint32_t vk = __shfl_sync(kFull, v, (t * kMbKB + lane) & 31);
+      const bool mine = lane < (uint32_t)kMbKB && vk != 0xffffffffu;
+      ring.issue(T + t, mine, mk.sk, 3 * mk.B, mk.sk + mk.det, kMbKB);
+      return slot_offsets(mk.sk, mk.sk + mk.det);
+    };
+    const uint32_t nb = min(BPG, (nbatch - it + nwarps - 1) / nwarps);
+    int my_res = 1;
+    uint64_t my_idx = 0;
+    offs = issue(0);
+    for (uint32_t t = 0; t < nb; ++t) {
+      const uint32_t offs_next = t + 1 < nb ? issue(t + 1) : 0u;
+      if (!landed(t, t + 1 < nb)) break;
+      const uint32_t v0 = (it + t * nwarps) * kMbKB, nm = min((uint32_t)kMbKB, V - v0);
+      const MbVert mk = mb_vert_shfl(me, (t * kMbKB + lane) & 31);
+      uint64_t idx;
+      const int res = mb_sample_batch(ring.slot(T + t, 0, kMbKB), ring.slot_bytes, ring.run_cap, offs, mk.B, mk.chk, nm,
+                                      t * kMbKB, &idx);
+      if (lane / kMbKB == t) {
+        my_res = res;
+        my_idx = idx;
+      }
+      if (lane < nm) {
+        const uint32_t *d = reinterpret_cast<const uint32_t *>(ring.slot(T + t, lane, kMbKB) + ring.run_cap + (offs >> 8));
+        reinterpret_cast<uint4 *>(q.det)[v0 + lane] = make_uint4(d[0], d[1], d[2], 0);
+      }
+      offs = offs_next;
+      __syncwarp();
+    }
+    if (failed) break;
+    T += nb;
+    if (v != 0xffffffffu) {
+      if (my_res == 1) q.rstate[2 * v] = 1;
+      mb_apply(my_res, my_idx, 0, me.g, b.graphs[me.g], b, q);
+    }
+    __syncwarp();
+  }
+  if (!sync()) return;
+
+  uint32_t round = 0;
+  while (__ldcg(q.go) == round + 1) {  // (the next round's marks come after its own barriers)
+    ++round;
+    if (round == 1) fence_proxy_async_all();  // det, written in round 0
+    ahead(gw);
+    for (uint32_t it = gw; it < nbatch && !failed; it += BPG * nwarps) {  // A
+      const uint32_t v = my_vertex(it), r0 = r_ahead, g = g_ahead;
+      ahead(it + BPG * nwarps);
+      uint32_t r = 0;
+      bool need = false;
+      MbVert me{};
+      if (v != 0xffffffffu) {
+        // L1 for the words that whole graphs and components share: nothing writes them in this phase,
+        // and L2 serves one line to everyone at the pace of one slice (7.4 -> 6.4 ms, see mark)
+        const bool act = __ldca(q.lastmod + g) == round && round < b.graphs[g].C;
+        if (act) {
+          const uint32_t p = __ldca(b.parent + r0);
+          const uint2 st = __ldca(reinterpret_cast<const uint2 *>(q.rstate) + r0);
+          r = p;
+          if (p != r0) {
+            r = dsu_find(b.parent, p);
+            b.label[v] = r;
+          }
+          need = !(p == r0 && st.x > st.y);  // a finished component is left out (see gz_query.cu)
+          if (need) me = mb_vert(b, v);
+        }
+      }
+      const uint32_t needm = __ballot_sync(kFull, need);
+      const uint32_t n = __popc(needm);
+      if (!n) continue;
+      uint32_t leader = 32;
+      if (need) leader = __ffs(__match_any_sync(needm, r)) - 1;
+      uint32_t rank = 0;
+      for (uint32_t mm = needm; mm; mm &= mm - 1) {
+        const uint32_t l = __ffs(mm) - 1, ll = __shfl_sync(kFull, leader, l);
+        rank += ll < leader || (ll == leader && l < lane);
+      }
+      if (need) perm[rank] = lane;
+      __syncwarp();
+      const uint32_t src = lane < n ? perm[lane] : 0u;
+      __syncwarp();
+      const uint32_t vq = __shfl_sync(kFull, v, src), rq = __shfl_sync(kFull, r, src);
+      const MbVert mq = mb_vert_shfl(me, src);  // member of lane
+      auto issue = [&](uint32_t t) {
+        const uint32_t m = (t * kMbKB + lane) & 31;
+        const MbVert mk = mb_vert_shfl(mq, m);
+        const uint32_t vm = __shfl_sync(kFull, vq, m);
+        const bool mine = lane < (uint32_t)kMbKB && t * kMbKB + lane < n;
+        ring.issue(T + t, mine, mk.sk + 3 * round * mk.B, 3 * mk.B, q.det + 4 * (size_t)(mine ? vm : 0), kMbKB);
+      };
+      const uint32_t nb = (n + kMbKB - 1) / kMbKB;
+      issue(0);
+      uint32_t acc[NW], dacc = 0, cur = 0xffffffffu, curW = 0;
+#pragma unroll
+      for (int k = 0; k < NW; ++k) acc[k] = 0;
+      auto flush = [&]() {
+        uint32_t *ac = q.racc + (uint64_t)cur * SW;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) {
+          const uint32_t wi = k * 32 + lane;
+          if (wi < curW && acc[k]) atomicXor(ac + wi, acc[k]);
+          acc[k] = 0;
+        }
+        if (lane < 3 && dacc) atomicXor(ac + curW + lane, dacc);
+        dacc = 0;
+      };
+      for (uint32_t t = 0; t < nb; ++t) {
+        if (t + 1 < nb) issue(t + 1);
+        if (!landed(t, t + 1 < nb)) break;
+#pragma unroll 1
+        for (uint32_t k = 0; k < (uint32_t)kMbKB && t * kMbKB + k < n; ++k) {
+          const uint32_t m = t * kMbKB + k;
+          const uint32_t c = __shfl_sync(kFull, rq, m), Bm = __shfl_sync(kFull, mq.B, m);
+          const uint32_t *sk = reinterpret_cast<const uint32_t *>(
+              __shfl_sync(kFull, reinterpret_cast<unsigned long long>(mq.sk), m));
+          if (c != cur) {
+            if (cur != 0xffffffffu) flush();
+            cur = c;
+            curW = 3 * Bm;
+          }
+          const uint8_t *slt = ring.slot(T + t, k, kMbKB);
+          const uint32_t *sl = bulk_run_at(slt, sk + 3 * round * Bm);
+          const uint32_t *sd = reinterpret_cast<const uint32_t *>(slt + ring.run_cap);
+#pragma unroll
+          for (int w = 0; w < NW; ++w) {
+            const uint32_t wi = w * 32 + lane;
+            if (wi < curW) acc[w] ^= sl[wi];
+          }
+          if (lane < 3) dacc ^= sd[lane];
+        }
+        __syncwarp();
+      }
+      if (failed) break;
+      T += nb;
+      flush();
+    }
+    if (!sync()) return;
+    fence_proxy_async_all();
+    ahead(gw);
+    for (uint32_t it = gw; it < nbatch && !failed; it += BPG * nwarps) {  // B
+      const uint32_t v = my_vertex(it), g = g_ahead;
+      bool root = v != 0xffffffffu && r_ahead == v;
+      ahead(it + BPG * nwarps);
+      if (root) {
+        // (a graph marked again in this phase reads round + 1: it took part all the same)
+        const uint32_t lm = __ldca(q.lastmod + g);
+        const uint2 st = __ldcg(reinterpret_cast<const uint2 *>(q.rstate) + v);
+        root = lm >= round && round < b.graphs[g].C && st.x <= st.y;
+      }
+      const uint32_t rootm = __ballot_sync(kFull, root);
+      const uint32_t n = __popc(rootm);
+      if (!n) continue;
+      if (root) perm[__popc(rootm & ((1u << lane) - 1u))] = lane;
+      __syncwarp();
+      const uint32_t src = lane < n ? perm[lane] : 0u;
+      __syncwarp();
+      const uint32_t vq = __shfl_sync(kFull, v, src), gq = __shfl_sync(kFull, g, src);
+      GraphDesc gd{};
+      uint64_t chk = 0;
+      if (lane < n) {
+        gd = b.graphs[gq];
+        chk = b.flip[gd.flip_off + gd.C];
+      }
+      auto issue = [&](uint32_t t) {
+        const uint32_t m = (t * kMbKB + lane) & 31;
+        const uint32_t vm = __shfl_sync(kFull, vq, m), Bm = __shfl_sync(kFull, gd.B, m);
+        const bool mine = lane < (uint32_t)kMbKB && t * kMbKB + lane < n;
+        const uint32_t *ac = q.racc + (uint64_t)(mine ? vm : 0) * SW;
+        ring.issue(T + t, mine, ac, 3 * Bm, ac + 3 * Bm, kMbKB);
+        return slot_offsets(ac, ac + 3 * Bm);
+      };
+      const uint32_t nb = (n + kMbKB - 1) / kMbKB;
+      int my_res = 1;
+      uint64_t my_idx = 0;
+      uint32_t offs = issue(0);
+      for (uint32_t t = 0; t < nb; ++t) {
+        const uint32_t offs_next = t + 1 < nb ? issue(t + 1) : 0u;
+        if (!landed(t, t + 1 < nb)) break;
+        const uint32_t nm = min((uint32_t)kMbKB, n - t * kMbKB), m = (t * kMbKB + lane) & 31;
+        uint64_t idx;
+        const int res = mb_sample_batch(ring.slot(T + t, 0, kMbKB), ring.slot_bytes, ring.run_cap, offs,
+                                        __shfl_sync(kFull, gd.B, m), __shfl_sync(kFull, (unsigned long long)chk, m),
+                                        nm, t * kMbKB, &idx);
+        if (lane / kMbKB == t) {
+          my_res = res;
+          my_idx = idx;
+        }
+        for (uint32_t k = 0; k < nm; ++k) {  // cleared for the next round
+          uint4 *ac = reinterpret_cast<uint4 *>(q.racc + (uint64_t)__shfl_sync(kFull, vq, t * kMbKB + k) * SW);
+          for (uint32_t i = lane; i < SW / 4; i += 32) ac[i] = make_uint4(0, 0, 0, 0);
+        }
+        offs = offs_next;
+        __syncwarp();
+      }
+      if (failed) break;
+      T += nb;
+      if (lane < n) {
+        if (my_res == 1) q.rstate[2 * vq] = round + 1;
+        mb_apply(my_res, my_idx, round, gq, gd, b, q);
+      }
+      __syncwarp();
+    }
+    if (!sync()) return;
+  }
+  for (uint32_t v0 = gw * 32; v0 < V; v0 += nwarps * 32) {
+    const uint32_t v = v0 + lane;
+    bool root = false;
+    uint32_t g = 0xffffffffu;
+    if (v < V) {
+      g = b.gov[v];
+      const uint32_t r = dsu_find(b.parent, __ldcg(b.label + v));
+      q.labels[v] = r - b.graphs[g].vbase;
+      root = r == v;
+    }
+    const uint32_t rm = __ballot_sync(kFull, root);
+    if (root) {
+      const uint32_t peers = __match_any_sync(rm, g);
+      if (lane == __ffs(peers) - 1) atomicAdd(q.ncc + g, (uint32_t)__popc(peers));
+    }
+  }
+}
+
 __global__ void k_mb_reset(uint32_t n, uint32_t *parent) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v < n) parent[v] = v;
@@ -1283,7 +1636,7 @@ struct gz_batch {
   uint64_t cap_worklist = 0;
   // capacities of the device tables (grown, never shrunk)
   uint64_t cap_graphs = 0, cap_tiles = 0, cap_V = 0, cap_bins = 0;
-  uint64_t cap_bv_V = 0, cap_bv_G = 0, cap_acc = 0;
+  uint64_t cap_bv_V = 0, cap_rounds_V = 0, cap_bv_G = 0, cap_acc = 0;
   gz::MBBufs captured{};    // buffers the captured Boruvka round was recorded with
   gz::MBBufs last_query{};  // buffers of the previous query
   GraphDesc *d_graphs = nullptr;
@@ -1309,6 +1662,11 @@ struct gz_batch {
   uint64_t *d_res = nullptr;
   uint32_t *d_res_g = nullptr;
   uint64_t cap_res = 0, cap_res_g = 0;
+  // one-launch query: accumulators; states and deterministic buckets (6 words a vertex); the results
+  // (ncc, lastmod) and control words, and the results on the host
+  uint32_t *d_racc = nullptr, *d_vstate = nullptr, *d_qres = nullptr, *h_qres = nullptr;
+  bool racc_dirty = true;  // d_racc may hold nonzero words
+  uint64_t cap_racc = 0, cap_vstate = 0, cap_qres = 0, cap_hqres = 0;
   uint32_t *d_order = nullptr, *d_order_comp = nullptr, *d_comp_start = nullptr, *d_ncomp = nullptr, *d_acc = nullptr;
   uint32_t *d_active = nullptr, *d_modified = nullptr, *d_round = nullptr, *d_ncc = nullptr;
   cudaGraphExec_t round_exec = nullptr;
@@ -1400,6 +1758,10 @@ void batch_destroy(gz_batch *h) {
   mb_free(h->d_modified);
   mb_free(h->d_round);
   mb_free(h->d_ncc);
+  mb_free(h->d_racc);
+  mb_free(h->d_vstate);
+  mb_free(h->d_qres);
+  if (h->h_qres) cudaFreeHost(h->h_qres);
   if (h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -1732,13 +2094,24 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
   return batch_flush_status(h);
 }
 
+int ensure_parent(gz_batch *h) {
+  const uint64_t V = h->total_V;
+  if (h->d_parent && h->d_label && h->cap_bv_V >= V) return GZ_OK;
+  const uint64_t Vn = headroom(h->cap_bv_V, V);
+  h->cap_bv_V = 0;
+  MB_TRY(mb_realloc_async(&h->d_parent, Vn, h->stream));
+  MB_TRY(mb_realloc_async(&h->d_label, Vn, h->stream));
+  h->cap_bv_V = Vn;
+  return GZ_OK;
+}
+
+// Buffers of the rounds driven from the host.
 int ensure_boruvka(gz_batch *h) {
   const uint64_t V = h->total_V, G = h->G;
-  if (!h->d_parent || h->cap_bv_V < V) {
-    const uint64_t Vn = headroom(h->cap_bv_V, V);
-    h->cap_bv_V = 0;
-    MB_TRY(mb_realloc_async(&h->d_parent, Vn, h->stream));
-    MB_TRY(mb_realloc_async(&h->d_label, Vn, h->stream));
+  MB_TRY(ensure_parent(h));
+  if (!h->d_cnt || h->cap_rounds_V < V) {
+    const uint64_t Vn = headroom(h->cap_rounds_V, V);
+    h->cap_rounds_V = 0;
     MB_TRY(mb_realloc_async(&h->d_cnt, Vn, h->stream));
     MB_TRY(mb_realloc_async(&h->d_fill, Vn, h->stream));
     MB_TRY(mb_realloc_async(&h->d_packed, Vn, h->stream));
@@ -1746,7 +2119,7 @@ int ensure_boruvka(gz_batch *h) {
     MB_TRY(mb_realloc_async(&h->d_order, Vn, h->stream));
     MB_TRY(mb_realloc_async(&h->d_order_comp, Vn, h->stream));
     MB_TRY(mb_realloc_async(&h->d_comp_start, Vn + 1, h->stream));
-    h->cap_bv_V = Vn;
+    h->cap_rounds_V = Vn;
   }
   const uint64_t slots = (V + kMbSpan - 1) / kMbSpan;
   MB_TRY(grow(&h->d_acc, h->cap_acc, (slots + 1) * (uint64_t)(h->max_B + 1) * 3, h->stream));
@@ -1790,8 +2163,120 @@ int enqueue_round(gz_batch *h, cudaStream_t s) {
   return GZ_OK;
 }
 
+// Buffers of the one-launch query. False: they do not fit, or the vertices are more than 2^21; the rounds of
+// batch_query_rounds then run. The line bounds the accumulators (about 350 to 500 B a vertex, 1 GB):
+// graphs of 1024 vertices, 2.05e6 together, take 2.8 ms in one launch and 4.4 in rounds, 1.02e6 1.5 and 2.5.
+constexpr uint64_t kMbOneLaunchMaxV = 1u << 21;
+constexpr uint32_t kQresCtl = 8;  // go, barrier
+bool one_launch_buffers(gz_batch *h) {
+  const uint64_t V = h->total_V;
+  if (V > kMbOneLaunchMaxV) return false;
+  int rc = ensure_parent(h);
+  const uint64_t had = h->d_racc ? h->cap_racc : 0;
+  if (rc == GZ_OK) rc = grow(&h->d_racc, h->cap_racc, V * racc_words(1, h->max_B), h->stream);
+  if (h->cap_racc != had) h->racc_dirty = true;
+  if (rc == GZ_OK) rc = grow(&h->d_vstate, h->cap_vstate, 6 * V + 4, h->stream);
+  if (rc == GZ_OK) rc = grow(&h->d_qres, h->cap_qres, 2 * (uint64_t)h->G + kQresCtl, h->stream);
+  if (rc == GZ_OK && (!h->h_qres || h->cap_hqres < 2 * (uint64_t)h->G)) {
+    const uint64_t n = headroom(h->cap_hqres, 2 * (uint64_t)h->G);
+    if (h->h_qres) cudaFreeHost(h->h_qres);
+    h->h_qres = nullptr;
+    h->cap_hqres = 0;
+    if (cudaMallocHost(&h->h_qres, 4 * n) != cudaSuccess) rc = GZ_ERR_CUDA;
+    else h->cap_hqres = n;
+  }
+  if (rc == GZ_OK) return true;
+  cudaGetLastError();
+  mb_free(h->d_racc);
+  mb_free(h->d_vstate);
+  h->cap_racc = h->cap_vstate = 0;
+  return false;
+}
+
+// One cooperative launch for every round of every graph, one synchronisation.
+int batch_query_launch(gz_batch *h, uint32_t *labels_out) {
+  const MBBufs b = h->bufs();
+  const uint32_t V = (uint32_t)h->total_V, G = h->G;
+  MbQuery q{};
+  q.rstate = h->d_vstate;
+  q.det = h->d_vstate + 2 * (((uint64_t)V + 1) & ~1ull);
+  q.racc = h->d_racc;
+  q.go = h->d_qres;
+  q.qbar = q.go + 1;
+  q.ncc = h->d_qres + kQresCtl;
+  q.lastmod = q.ncc + G;
+  q.labels = h->d_label;
+  q.sw = racc_words(1, h->max_B);
+  q.G = G;
+  auto *kern = h->max_B <= 42 ? k_mb_query<4> : k_mb_query<Region<1>::kNW>;
+  MB_CUDA(smem_optin(kern));
+  int optin = 0;
+  cudaFuncAttributes fa{};
+  MB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+  MB_CUDA(cudaFuncGetAttributes(&fa, kern));
+  const size_t warp_smem = bv_warp_bytes(mbq_ring_words(b.acc_words), kMbKB);
+  const int max_warps = (int)((optin - (int)fa.sharedSizeBytes) / warp_smem);
+  // a warp per batch of vertices while there are batches for it, one block per SM
+  const uint32_t nbatch = (V + kMbKB - 1) / kMbKB;
+  const int want = (int)cdiv(nbatch, num_sms());
+  const int warps = std::min(std::max(want, 2), std::min(kMbqMaxThreads / 32, max_warps));
+  const int blocks = std::min<int>(num_sms(), (int)cdiv(nbatch, warps));
+  MB_CUDA(cudaMemsetAsync(q.qbar, 0, sizeof(uint32_t), h->stream));
+  // a query that ran to its end leaves every accumulator zero
+  if (h->racc_dirty) MB_CUDA(cudaMemsetAsync(h->d_racc, 0, sizeof(uint32_t) * h->cap_racc, h->stream));
+  h->racc_dirty = true;
+  MBBufs a_b = b;
+  void *args[] = {&a_b, &q};
+  MB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(blocks), dim3(32 * warps), args,
+                                      warps * warp_smem, h->stream));
+  h->launches++;
+  MB_CUDA(cudaMemcpyAsync(h->h_qres, q.ncc, sizeof(uint32_t) * 2 * G, cudaMemcpyDeviceToHost, h->stream));
+  if (labels_out)
+    MB_CUDA(cudaMemcpyAsync(labels_out, h->d_label, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost, h->stream));
+  return GZ_OK;
+}
+
+int batch_query_rounds(gz_batch *h, uint32_t *labels_out);
+
 // boruvka_emulation for every graph at once; per graph the rounds stop independently.
 int batch_query(gz_batch *h, uint32_t *labels_out) {
+  if (!one_launch_buffers(h)) return batch_query_rounds(h, labels_out);
+  const uint32_t G = h->G;
+  cudaEvent_t q0 = nullptr, q1 = nullptr;
+  if (h->prof) {
+    cudaEventCreate(&q0);
+    cudaEventCreate(&q1);
+    cudaEventRecord(q0, h->stream);
+  }
+  int rc = batch_query_launch(h, labels_out);
+  if (h->prof) cudaEventRecord(q1, h->stream);
+  const int rc_flush = batch_flush_status(h);
+  if (rc == GZ_OK) rc = rc_flush;
+  if (h->prof) {
+    float ms = 0;
+    if (rc == GZ_OK && cudaEventElapsedTime(&ms, q0, q1) == cudaSuccess) h->prof_query_ms += ms;
+    cudaEventDestroy(q0);
+    cudaEventDestroy(q1);
+  }
+  if (rc == GZ_OK || rc == GZ_ERR_BAD_SAMPLE) {
+    h->racc_dirty = false;
+    h->ncc.assign(h->h_qres, h->h_qres + G);
+    h->rounds.assign(h->h_qres + G, h->h_qres + 2 * (size_t)G);
+    h->status.assign(G, GZ_OK);
+    uint32_t ran = 0;
+    for (uint32_t g = 0; g < G; ++g) {
+      const uint32_t C = h->graphs[g].C;
+      if (h->rounds[g] >= C) h->status[g] = GZ_ERR_OUT_OF_SAMPLES;
+      ran = std::max(ran, std::min(h->rounds[g], C - 1));
+    }
+    h->prof_rounds += ran;
+  }
+  return rc;
+}
+
+// The same in rounds driven from the host, members grouped by component in each: for more vertices
+// than the one launch takes, and where its buffers do not fit.
+int batch_query_rounds(gz_batch *h, uint32_t *labels_out) {
   MB_TRY(ensure_boruvka(h));
   const MBBufs b = h->bufs();
   const size_t V = h->total_V;

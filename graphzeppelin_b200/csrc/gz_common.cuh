@@ -558,6 +558,93 @@ static __device__ bool dsu_unite(uint32_t *parent, uint32_t a, uint32_t b) {
   }
 }
 
+// ---- one-launch queries (gz_query.cu, gz_batch.cu) ----------------------------------------------
+__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Barrier over every block of the launch. CL: the launch is one cluster (hardware barrier; threads
+// that have exited are not waited for). Otherwise the blocks of a cooperative launch count their
+// arrivals in *count (zeroed before the launch); barrier number k completes at k * gridDim.x
+// arrivals. Writes before it are seen by every block after it (release at the arrival, acquire
+// after it). A block with a failed warp (failed = true in any thread) leaves without arriving; a
+// block that waits longer than kWaitLimitNs sets the timeout status. Both return false, and the
+// caller returns from the kernel (the other blocks then time out at their next barrier).
+template <bool CL>
+__device__ bool launch_barrier(uint32_t *count, uint32_t k, bool failed, uint32_t *status) {
+  if (__syncthreads_or(failed)) return false;
+  if (CL) {
+    __threadfence();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  }
+  __shared__ uint32_t s_ok;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(count, 1u);
+    const uint32_t target = k * gridDim.x;
+    uint32_t ok = 1;
+    if (ld_acquire_gpu(count) < target) {
+      const uint64_t t0 = global_ns();
+      while (ld_acquire_gpu(count) < target) {
+        if (global_ns() - t0 > kWaitLimitNs) {
+          atomicOr(status, kStatusTimeout);
+          ok = 0;
+          break;
+        }
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// Generic-proxy writes of other threads, made visible by the barrier above, before this thread's
+// bulk copies (async proxy) read them.
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Roots of x and y, both chains followed together (path halving, as dsu_find).
+__device__ __forceinline__ void find_two(uint32_t *parent, uint32_t &x, uint32_t &y) {
+  bool go_x = true, go_y = x != y;
+  if (!go_y) y = x;
+  while (go_x || go_y) {
+    const uint32_t px = go_x ? __ldcg(parent + x) : x, py = go_y ? __ldcg(parent + y) : y;
+    const uint32_t gx = px != x ? __ldcg(parent + px) : x, gy = py != y ? __ldcg(parent + py) : y;
+    if (px == x) go_x = false;
+    else if (gx == px) x = px, go_x = false;
+    else __stcg(parent + x, gx), x = gx;
+    if (py == y) go_y = false;
+    else if (gy == py) y = py, go_y = false;
+    else __stcg(parent + y, gy), y = gy;
+  }
+}
+
+// Unites the trees of x and y (vertices of a graph whose ids start at vbase): the root of lower rank is
+// linked under the other (x = parent, y = child on return). False: one tree already.
+__device__ __forceinline__ bool unite_two(uint32_t *parent, uint32_t &x, uint32_t &y, uint32_t vbase) {
+  for (;;) {
+    find_two(parent, x, y);
+    if (x == y) return false;
+    if (rank_of(x - vbase) < rank_of(y - vbase)) {
+      const uint32_t t = x;
+      x = y;
+      y = t;
+    }
+    if (atomicCAS(parent + y, y, x) == y) return true;
+  }
+}
+
+__device__ __forceinline__ uint32_t slot_offsets(const uint32_t *run, const uint32_t *det) {
+  return ((uint32_t)(uintptr_t)run & 15u) | (((uint32_t)(uintptr_t)det & 15u) << 8);
+}
+
+// Words of one root's accumulator: CPS B column buckets, the deterministic bucket, padded to 16 B.
+__host__ __device__ inline uint32_t racc_words(uint32_t cps, uint32_t B) { return (3 * (cps * B + 1) + 3) & ~3u; }
+
 // Sketch::sample (src/sketch.cpp:94-116) on one merged column held one or two buckets per lane
 // (lane j holds bucket j and j + 32) plus the deterministic bucket (same on every lane).
 __device__ __forceinline__ int warp_sample(const uint32_t (&d)[3], const uint32_t (&a)[2][3],
