@@ -341,7 +341,9 @@ class CCSketchAlg:
 
     def apply_update_batch(self, thr_id: int, src_vertex: int, dst_vertices: Sequence[int]) -> None:
         d = np.ascontiguousarray(dst_vertices, dtype=np.uint32)
-        _check(self.lib.gz_apply_update_batch(self._h, thr_id, src_vertex, _ptr(d), d.size))
+        rc = self.lib.gz_apply_update_batch(self._h, thr_id, src_vertex, d.ctypes.data, d.size)
+        if rc:
+            _check(rc)
 
     def has_cached_query(self, query_code: int) -> bool:
         out = ctypes.c_int()

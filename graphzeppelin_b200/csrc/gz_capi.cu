@@ -375,11 +375,11 @@ int choose_planes(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tp
     if (asked) return fail(GZ_ERR_INVALID, "coded entries take tiles of 4 to 32 vertices, 1 to 8 per bin");
     return GZ_OK;
   }
-  // By default past 2^18 vertices the pipelined staged kernel stays in use (large sparse graphs,
-  // where a wave brings few entries per tile)
+  // By default past 2^18 vertices entries stay plain (large sparse graphs, where a wave brings few
+  // entries per tile) and are hashed where they are applied
   if (!asked && h->V > kPlaneDefaultMaxV) return GZ_OK;
   // Tiles of 32 vertices, fewer where that leaves SMs without a tile or two (a call is then as long as
-  // its last wave: 1,024 vertices, 8,528 records: 18 us in tiles of 32, 9 us in tiles of 8)
+  // its last wave: 1,024 vertices, 8,528 records: 18 us in tiles of 32, 11 us in tiles of 8)
   uint32_t shift = vpt_req ? (uint32_t)__builtin_ctz(vpt_req) : 5;
   while (!vpt_req && !tpb_req && !threads_req && shift > 3 && (h->V >> shift) < 2u * gz::num_sms()) --shift;
   uint32_t bshift = shift;
@@ -463,7 +463,7 @@ int choose_tiling(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tp
   // Left to itself, a handle without coded entries applies its plain entries through bucket planes:
   // tiles of 8 vertices (four CTAs an SM) with a gutter bin each, of 16 or 32 where that many more
   // vertices still keep the bins within the shared-memory sort. Against staging whole tiles: 2^20
-  // vertices, 1.28e7 records 5.5 -> 4.5 ms; CubeSketch, 5,003 vertices, 1e6 records 3.7 -> 0.54 ms.
+  // vertices, 1.28e7 records 5.5 -> 2.8 ms; CubeSketch, 5,003 vertices, 1e6 records 3.7 -> 0.47 ms.
   if (!h->in_place && h->planes_mode < 0 && h->pipe_mode < 0 && !vpt_req && !threads_req && !tpb_req &&
       h->C <= gz::kPlaneMaxColumnsWide) {
     shift = 3;
@@ -750,22 +750,39 @@ int push_staged_entries(gz_alg *h) {
   return GZ_OK;
 }
 
-int stage_entry(gz_alg *h, uint32_t v, uint32_t w) {
-  if (!h->h_ent[0]) {
-    for (int i = 0; i < 2; ++i) {
-      GZ_TRY(host_alloc(&h->h_ent[i], kEntStage));
-      GZ_CUDA(cudaEventCreateWithFlags(&h->ev_ent_done[i], cudaEventDisableTiming));
-      GZ_CUDA(cudaEventRecord(h->ev_ent_done[i], h->stream));
-    }
+int stage_ensure(gz_alg *h) {
+  if (h->h_ent[0]) return GZ_OK;
+  for (int i = 0; i < 2; ++i) {
+    GZ_TRY(host_alloc(&h->h_ent[i], kEntStage));
+    GZ_CUDA(cudaEventCreateWithFlags(&h->ev_ent_done[i], cudaEventDisableTiming));
+    GZ_CUDA(cudaEventRecord(h->ev_ent_done[i], h->stream));
   }
-  h->h_ent[h->h_ent_cur][h->h_ent_n++] = make_uint2(v, w);
-  if (h->h_ent_n == kEntStage) GZ_TRY(push_staged_entries(h));
   return GZ_OK;
 }
 
-int check_status(gz_alg *h) {
+// Entries (v, w[0 .. n)) written to the staging buffer a run at a time (a loop the compiler turns into
+// vector stores), pushed whenever it is full.
+int stage_entries(gz_alg *h, uint32_t v, const uint32_t *w, size_t n) {
+  GZ_TRY(stage_ensure(h));
+  while (n) {
+    const size_t run = std::min<size_t>(n, kEntStage - h->h_ent_n);
+    uint64_t *out = reinterpret_cast<uint64_t *>(h->h_ent[h->h_ent_cur] + h->h_ent_n);
+    for (size_t i = 0; i < run; ++i) out[i] = ((uint64_t)w[i] << 32) | v;
+    h->h_ent_n += run;
+    w += run;
+    n -= run;
+    if (h->h_ent_n == kEntStage) GZ_TRY(push_staged_entries(h));
+  }
+  return GZ_OK;
+}
+
+int status_enqueue(gz_alg *h) {
   GZ_CUDA(cudaMemcpyAsync(h->h_status, h->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-  GZ_CUDA(cudaStreamSynchronize(h->stream));
+  return GZ_OK;
+}
+
+// The status that status_enqueue copied, once the stream has been waited for.
+int status_result(gz_alg *h) {
   const uint32_t st = h->h_status[0] | h->deferred_status;
   h->deferred_status = 0;
   if (st) {
@@ -778,11 +795,16 @@ int check_status(gz_alg *h) {
   return GZ_OK;
 }
 
+int check_status(gz_alg *h) {
+  GZ_TRY(status_enqueue(h));
+  GZ_CUDA(cudaStreamSynchronize(h->stream));
+  return status_result(h);
+}
+
 int flush_all(gz_alg *h) {
   GZ_TRY(push_staged_entries(h));
   GZ_TRY(apply_pending(h));
-  GZ_CUDA(cudaStreamSynchronize(h->stream));
-  return check_status(h);
+  return check_status(h);  // (its synchronisation is the flush's)
 }
 
 int check_unlocked(gz_alg *h) {
@@ -1044,6 +1066,7 @@ int run_boruvka(gz_alg *h) {
   GZ_TRY(boruvka_enqueue(h, h->qgraph, h->bgeom(), h->d_sk, h->bv, h->d_final, h->d_ncc, h->h_qpin,
                          h->stream));
   h->prof_end(pi, 2);
+  GZ_TRY(status_enqueue(h));
   GZ_CUDA(cudaStreamSynchronize(h->stream));
   boruvka_account(h->qgraph, h->h_qpin, query_mode_of(h) == 1);
   const uint32_t round = h->h_qpin[0];
@@ -1052,7 +1075,7 @@ int run_boruvka(gz_alg *h) {
     return fail(GZ_ERR_OUT_OF_SAMPLES, out_of_samples_msg(h, round));
   }
   h->prof_acc.query_rounds += round + 1;
-  GZ_TRY(check_status(h));
+  GZ_TRY(status_result(h));
   h->last_ncc = h->h_qpin[2];
   h->last_rounds = round;
   h->dsu_valid = true;
@@ -1336,12 +1359,11 @@ int gz_apply_update_batch(gz_alg_t *h, int, uint32_t src, const uint32_t *dsts, 
   GZ_TRY(check_unlocked(h));
   if (!h->eager) invalidate_answer(h);
   if (src >= h->V) return fail(GZ_ERR_BAD_VERTEX, "src vertex id >= V");
-  for (size_t i = 0; i < n; ++i) {
-    if (dsts[i] >= h->V) return fail(GZ_ERR_BAD_VERTEX, "dst vertex id >= V");
-  }
+  uint32_t most = 0;
+  for (size_t i = 0; i < n; ++i) most = dsts[i] > most ? dsts[i] : most;
+  if (n && most >= h->V) return fail(GZ_ERR_BAD_VERTEX, "dst vertex id >= V");
   h->symmetric = false;  // one endpoint's sketch only
-  for (size_t i = 0; i < n; ++i) GZ_TRY(stage_entry(h, src, dsts[i]));
-  return GZ_OK;
+  return stage_entries(h, src, dsts, n);
 }
 
 int gz_apply_raw_buckets_update(gz_alg_t *h, uint32_t src, const void *raw) {
@@ -1364,8 +1386,8 @@ int gz_update(gz_alg_t *h, uint32_t src, uint32_t dst, int) {
   GZ_TRY(check_unlocked(h));
   pre_insert_one(h, src, dst);  // CCSketchAlg::update calls pre_insert first
   if (src >= h->V || dst >= h->V) return fail(GZ_ERR_BAD_VERTEX, "vertex id >= V");
-  GZ_TRY(stage_entry(h, src, dst));
-  GZ_TRY(stage_entry(h, dst, src));
+  GZ_TRY(stage_entries(h, src, &dst, 1));
+  GZ_TRY(stage_entries(h, dst, &src, 1));
   return GZ_OK;
 }
 
