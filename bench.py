@@ -228,7 +228,7 @@ def roofline(alg, n, prof, steps, ingest_ms, hash_peak, hbm_peak_gbs, update_pea
         coded = C  # every column hashed once per record in the gutter pass
         g_bytes = 9 * n + 9 * n + 2 * n * 16
         kernels["gutter"] = {
-            "kernels": "k_gutter (count) + k_hash_sort_scatter", "launch_ms": t_g * 1e3,
+            "kernels": "k_count_records + k_hash_sort_scatter", "launch_ms": t_g * 1e3,
             "bound": "int", "hashes_per_launch": n * coded,
             "int": {"achieved": n * coded / t_g / 1e9, "peak": hash_peak / 1e9, "unit": "Ghash/s",
                     "frac": n * coded / t_g / hash_peak},
@@ -251,7 +251,7 @@ def roofline(alg, n, prof, steps, ingest_ms, hash_peak, hbm_peak_gbs, update_pea
                     "frac": u_bytes / t_u / 1e9 / hbm_peak_gbs, "bytes_per_launch": u_bytes}}
     else:
         kernels["gutter"] = {"kernels": "k_gutter (count) + k_gutter_sort_scatter", "launch_ms": t_g * 1e3}
-        kernels["sketch_update"] = {"kernels": "k_sketch_update (staged tiles, hashed per endpoint)",
+        kernels["sketch_update"] = {"kernels": "k_plane_update (plain entries, hashed per endpoint)",
                                     "launch_ms": t_u * 1e3, "hashes_per_launch": 2 * n * (C + 1),
                                     "int": {"achieved": 2 * n * (C + 1) / t_u / 1e9,
                                             "frac": 2 * n * (C + 1) / t_u / hash_peak}}

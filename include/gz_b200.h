@@ -294,8 +294,8 @@ GZ_API int gz_measure_update_rate(int repeats, double *updates_per_s);
 /* Tuning knobs of the ingest kernels (0 picks the default): vertices per shared-memory tile
  * (power of two in [4, 64]; at most 32 with coded entries), threads per block of the
  * sketch-update kernel, tiles per gutter bin (power of two <= 64; 1 with coded entries), and the
- * gutter entry form for records: 1 = plain entries {vertex, neighbour} (hashed per endpoint by a
- * staged-tile sketch-update kernel), 2 = coded entries (each record hashed once in the gutter into
+ * gutter entry form for records: 1 = plain entries {vertex, neighbour} (hashed per endpoint by the
+ * sketch update), 2 = coded entries (each record hashed once in the gutter into
  * per-column depth codes, applied through bucket planes; CameoSketch with at most 31 columns and
  * at most 8192 gutter bins; 4-bit codes where they fit a 16-byte entry, else 3-bit codes),
  * 3 = coded entries with 3-bit codes (code 7 = depth 7 or more, hashed again where applied).
@@ -329,7 +329,7 @@ GZ_API int gz_set_pipeline(gz_alg_t *alg, int mode);
  * A gz_batch_t holds num_graphs independent CCSketchAlg instances (each its own V, seed and
  * sketch geometry, include/cc_sketch_alg.h:69) in one device allocation. One ingest call runs one
  * gutter pass and ONE persistent sketch-update launch over the tiles of every graph; one query
- * runs Boruvka for all graphs at once, each round a replayed CUDA graph, each graph stopping on
+ * runs Boruvka for all graphs at once in one launch (up to 2^21 vertices together), each graph stopping on
  * its own. Per graph the sketches, partition, last_query_rounds and out-of-samples outcome equal
  * those of a gz_alg_t with the same V and seed fed the same records. */
 typedef struct gz_batch gz_batch_t;
@@ -365,7 +365,8 @@ GZ_API int gz_batch_load_sketches(gz_batch_t *batch, uint32_t graph, const void 
 /* Shape of the batched sketch-update launch: threads per CTA (multiple of 32 in [64, 1024]),
  * CTAs sharing one SM (1..4, threads * CTAs <= 2048; each CTA stages its tiles in 1/ctas of the
  * SM's shared memory, so one CTA's bulk copies overlap another's XORs), and vertices per tile per
- * graph (NULL or 0 = the largest power of two <= 64 that fits). 0 picks the default (1024, 1).
+ * graph (NULL or 0 = the largest power of two <= 64 that fits). 0 picks the default (1024, 1), with which
+ * graphs of at most 31 columns and no vertices per tile asked for are applied through bucket planes.
  * Sketch contents are kept; only the tiling changes. */
 GZ_API int gz_batch_set_tuning(gz_batch_t *batch, uint32_t threads_per_block, uint32_t ctas_per_sm,
                                const uint32_t *vertices_per_tile);
