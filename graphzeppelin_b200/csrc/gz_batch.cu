@@ -2163,10 +2163,12 @@ int enqueue_round(gz_batch *h, cudaStream_t s) {
   return GZ_OK;
 }
 
-// Buffers of the one-launch query. False: they do not fit, or the vertices are more than 2^21; the rounds of
-// batch_query_rounds then run. The line bounds the accumulators (about 350 to 500 B a vertex, 1 GB):
-// graphs of 1024 vertices, 2.05e6 together, take 2.8 ms in one launch and 4.4 in rounds, 1.02e6 1.5 and 2.5.
-constexpr uint64_t kMbOneLaunchMaxV = 1u << 21;
+// Buffers of the one-launch query. False: they do not fit, or the vertices are more than 2^23; the rounds of
+// batch_query_rounds then run. The line bounds the accumulators (about 350 to 500 B a vertex, 4 GB) and
+// their one allocation (a handle's first query of 8.2e6 vertices takes 22 ms against 18 in rounds). Graphs
+// of 1024 vertices, launch against rounds: 1.02e6 vertices together 1.5 and 2.5 ms, 2.05e6 2.8 and 4.3,
+// 4.1e6 5.4 and 7.7, 8.2e6 10.8 and 14.7.
+constexpr uint64_t kMbOneLaunchMaxV = 1u << 23;
 constexpr uint32_t kQresCtl = 8;  // go, barrier
 bool one_launch_buffers(gz_batch *h) {
   const uint64_t V = h->total_V;

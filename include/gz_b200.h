@@ -329,7 +329,7 @@ GZ_API int gz_set_pipeline(gz_alg_t *alg, int mode);
  * A gz_batch_t holds num_graphs independent CCSketchAlg instances (each its own V, seed and
  * sketch geometry, include/cc_sketch_alg.h:69) in one device allocation. One ingest call runs one
  * gutter pass and ONE persistent sketch-update launch over the tiles of every graph; one query
- * runs Boruvka for all graphs at once in one launch (up to 2^21 vertices together), each graph stopping on
+ * runs Boruvka for all graphs at once in one launch (up to 2^23 vertices together), each graph stopping on
  * its own. Per graph the sketches, partition, last_query_rounds and out-of-samples outcome equal
  * those of a gz_alg_t with the same V and seed fed the same records. */
 typedef struct gz_batch gz_batch_t;

@@ -1,4 +1,4 @@
-"""The batched query's two forms (one launch up to 2^21 vertices, grouping rounds beyond) and batches
+"""The batched query's two forms (one launch up to 2^23 vertices, grouping rounds beyond) and batches
 whose graphs take different sketch-update forms give what each graph gives alone."""
 import numpy as np
 import pytest
@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 def test_grouping_rounds_equal_one_launch(gz):
     from graphzeppelin_b200 import streams as S
-    V, n = 1024, 2100  # 2.15e6 vertices together; halves below 2^21
+    V, n = 1024, 8200  # 8.4e6 vertices together; halves below 2^23
     kinds = [S.planted_partition_stream(V, k, 7 + k, mean_degree=6, min_size=5)[0].records for k in (1, 9, 60)]
     kinds.append(np.zeros(0, dtype=S.RECORD_DTYPE))
     sts = [kinds[i % 4] for i in range(n)]
