@@ -269,11 +269,11 @@ struct gz_alg {
     g.direct_max = cube || g.groups > 1 ? 0 : (uint32_t)std::min(even * direct_factor, 4.0e9);
     return g;
   }
-  // Records of one call that go straight to the sketches: when the call brings so few that most of
-  // its tiles would be updated in place anyway, one launch without a gutter does it.
-  bool direct_call(uint64_t n) const {
+  // Whether the n records of a call go straight to the sketches: one launch without a gutter.
+  gz::DirectRoute direct;
+  bool direct_call(uint64_t n) {
     if (cube || C > gz::kPlaneMaxColumns || !(planes || plain_planes)) return false;
-    return 2.0 * (double)n < (double)pgeom().direct_max * ntiles;
+    return direct.take(n, (double)pgeom().direct_max * ntiles, entries_pending, (uint64_t)V * sketch_bytes);
   }
   gz::BoruvkaGeom bgeom() const {
     gz::BoruvkaGeom g;
@@ -804,6 +804,7 @@ int check_status(gz_alg *h) {
 int flush_all(gz_alg *h) {
   GZ_TRY(push_staged_entries(h));
   GZ_TRY(apply_pending(h));
+  h->direct.flushed();
   return check_status(h);  // (its synchronisation is the flush's)
 }
 
@@ -1470,6 +1471,7 @@ int gz_query_submit(gz_alg_t *h, uint64_t *ticket) {
   // every update so far goes to the stream ahead of the query; nothing waits here
   GZ_TRY(push_staged_entries(h));
   GZ_TRY(apply_pending(h));
+  h->direct.flushed();
   GZ_TRY(tickets_ensure(h));
   auto &T = h->tq;
   gz_alg::Ticket t;
@@ -1706,6 +1708,7 @@ int gz_clear(gz_alg_t *h) {
   h->nchunks = 0;
   h->gutter_used = 0;
   h->entries_pending = 0;
+  h->direct.flushed();
   h->h_ent_n = 0;
   const uint64_t v_pad = ((uint64_t)h->V + 63) & ~63ull;
   GZ_CUDA(cudaMemsetAsync(h->d_sk, 0, v_pad * h->sketch_bytes, h->stream));
