@@ -992,7 +992,7 @@ int boruvka_enqueue(gz_alg *h, gz::BoruvkaGraph &q, const gz::BoruvkaGeom &g, co
                     cudaStream_t s) {
   GZ_TRY(bv_ensure_mode(h, b, s));
   const int mode = query_mode_of(h);
-  if (mode == 2) GZ_CUDA(gz::boruvka_query_launch(g, h->samples, sk, b, 0, d_final, d_ncc, s));
+  if (mode == 2) GZ_CUDA(gz::boruvka_query_launch(g, h->samples, sk, b, d_final, d_ncc, s));
   else if (mode == 1) GZ_CUDA(gz::boruvka_graph_launch(q, g, h->samples, sk, b, d_final, d_ncc, s));
   else GZ_CUDA(gz::boruvka_host_loop(g, h->samples, sk, b, d_final, d_ncc, pin, s));
   GZ_CUDA(cudaMemcpyAsync(pin, b.ctl, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -314,11 +314,10 @@ cudaError_t boruvka_host_loop(const BoruvkaGeom &g, uint32_t samples, const uint
 
 // boruvka_emulation in one kernel launch (gz_query.cu; all rounds on the device, barriers over the
 // launch between the phases of a round): the same answer, rounds, samples and trace as the graph
-// and the host loop. b.ctl then holds the rounds and the out-of-samples flag. When *b.status has
-// a bit of abort_mask set as the kernel starts, the query is not run and nothing is written.
+// and the host loop. b.ctl then holds the rounds and the out-of-samples flag.
 cudaError_t boruvka_query_launch(const BoruvkaGeom &g, uint32_t samples, const uint8_t *sketches,
-                                 const BoruvkaBufs &b, uint32_t abort_mask, uint32_t *labels_out,
-                                 uint32_t *ncc, cudaStream_t s);
+                                 const BoruvkaBufs &b, uint32_t *labels_out, uint32_t *ncc,
+                                 cudaStream_t s);
 size_t query_racc_words(uint32_t V, uint32_t cps, uint32_t B);  // words of BoruvkaBufs::racc
 
 int num_sms();

@@ -123,16 +123,13 @@ constexpr uint32_t kMinRingWords = 29;  // a warp's stage (3 words more) holds i
 template <int CPS, int NW, int KB, bool CL>
 __global__ void __launch_bounds__(kBvqMaxThreads<CPS>, 1)
 k_bv_query(BoruvkaGeom g, const uint32_t *__restrict__ sk_words, BoruvkaBufs b, uint32_t samples,
-           uint32_t abort_mask, uint32_t *labels_out, uint32_t *ncc) {
+           uint32_t *labels_out, uint32_t *ncc) {
   extern __shared__ __align__(16) uint8_t bv_smem[];
-  __shared__ uint32_t s_word[2];
+  __shared__ uint32_t s_big;
   constexpr uint32_t BPG = 32 / KB;  // batches per 32 vertices
   const uint32_t V = g.V, tid = threadIdx.x, lane = tid & 31;
   const uint32_t W = 3 * CPS * g.B, SW = racc_words(CPS, g.B), detw = 3 * g.C * g.B;
   const uint32_t ring_words = max(W, kMinRingWords);
-  if (tid == 0) s_word[0] = __ldcg(b.status);
-  __syncthreads();
-  if (s_word[0] & abort_mask) return;  // an earlier update failed: the query is not run
   BvRing ring;
   ring.init(bv_smem + (tid >> 5) * bv_warp_bytes(ring_words, KB), ring_words, KB);
   uint32_t *perm = ring.stage;  // 32 words: the warp's vertices in processing order
@@ -261,10 +258,10 @@ k_bv_query(BoruvkaGeom g, const uint32_t *__restrict__ sk_words, BoruvkaBufs b, 
         const uint32_t votes = __popc(__match_any_sync(kFull, p));
         const uint32_t m = __ballot_sync(kFull, votes >= 17);
         const uint32_t most = __shfl_sync(kFull, p, m ? __ffs(m) - 1 : 0);
-        if (lane == 0) s_word[1] = m ? most : 0xffffffffu;
+        if (lane == 0) s_big = m ? most : 0xffffffffu;
       }
       __syncthreads();
-      big = s_word[1];
+      big = s_big;
     }
     const bool skip_done = big == 0xffffffffu && !trace;
     uint32_t cpl[NW], dcpl = 0;
@@ -468,8 +465,8 @@ constexpr int kClusterThreads = 512;
 size_t query_racc_words(uint32_t V, uint32_t cps, uint32_t B) { return (size_t)V * racc_words(cps, B); }
 
 cudaError_t boruvka_query_launch(const BoruvkaGeom &g, uint32_t samples, const uint8_t *sketches,
-                                 const BoruvkaBufs &b, uint32_t abort_mask, uint32_t *labels_out,
-                                 uint32_t *ncc, cudaStream_t s) {
+                                 const BoruvkaBufs &b, uint32_t *labels_out, uint32_t *ncc,
+                                 cudaStream_t s) {
   const uint32_t *sk = reinterpret_cast<const uint32_t *>(sketches);
   auto warp_bytes = [&](uint32_t KB) {
     return (size_t)bv_warp_bytes(std::max(3 * g.cps * g.B, kMinRingWords), (int)KB);
@@ -497,7 +494,7 @@ cudaError_t boruvka_query_launch(const BoruvkaGeom &g, uint32_t samples, const u
       at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
       cfg.attrs = at;
       cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, kern_cluster, g, sk, b, samples, abort_mask, labels_out, ncc);
+      e = cudaLaunchKernelEx(&cfg, kern_cluster, g, sk, b, samples, labels_out, ncc);
       if (e == cudaSuccess) {
         add_launches(1);
         return e;
@@ -524,9 +521,9 @@ cudaError_t boruvka_query_launch(const BoruvkaGeom &g, uint32_t samples, const u
     BoruvkaGeom a_g = g;
     const uint32_t *a_sk = sk;
     BoruvkaBufs a_b = b;
-    uint32_t a_samples = samples, a_mask = abort_mask;
+    uint32_t a_samples = samples;
     uint32_t *a_labels = labels_out, *a_ncc = ncc;
-    void *args[] = {&a_g, &a_sk, &a_b, &a_samples, &a_mask, &a_labels, &a_ncc};
+    void *args[] = {&a_g, &a_sk, &a_b, &a_samples, &a_labels, &a_ncc};
     // every block resident at once (the launch fails otherwise): a barrier never waits for a block
     // that has not started
     e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(blocks), dim3(threads), args,
