@@ -1069,9 +1069,11 @@ int run_boruvka(gz_alg *h) {
   h->prof_end(pi, 2);
   GZ_TRY(status_enqueue(h));
   GZ_CUDA(cudaStreamSynchronize(h->stream));
+  const gz::QueryOutcome outcome = gz::query_outcome(h->h_status[0], h->h_qpin[1]);
+  if (outcome == gz::QueryOutcome::kTimeout) return status_result(h);
   boruvka_account(h->qgraph, h->h_qpin, query_mode_of(h) == 1);
   const uint32_t round = h->h_qpin[0];
-  if (h->h_qpin[1]) {
+  if (outcome == gz::QueryOutcome::kOutOfSamples) {
     h->last_rounds = round;
     return fail(GZ_ERR_OUT_OF_SAMPLES, out_of_samples_msg(h, round));
   }
@@ -1525,20 +1527,25 @@ int gz_query_wait(gz_alg_t *h, uint64_t ticket, uint32_t *parent_out, uint32_t *
     h->tq.pool.push_back(t);
     return fail(GZ_ERR_CUDA, cudaGetErrorString(e));
   }
-  boruvka_account(h->tq.graph, t.pin, t.graph);
-  const uint32_t round = t.pin[0], oos = t.pin[1], ncc = t.pin[2], st = t.pin[3];
+  const uint32_t round = t.pin[0], ncc = t.pin[2], st = t.pin[3];
+  const gz::QueryOutcome outcome = gz::query_outcome(st, t.pin[1]);
   // bits of updates submitted before the query are reported by the next flush, as usual
   h->deferred_status |= st & (gz::kStatusBadVertex | gz::kStatusTimeout);
-  if (rounds) *rounds = round;
   int rc = GZ_OK;
-  if (oos) {
-    rc = fail(GZ_ERR_OUT_OF_SAMPLES, out_of_samples_msg(h, round));
-  } else if (st & gz::kStatusBadSample) {
-    rc = fail(GZ_ERR_BAD_SAMPLE, "a sampled edge decoded to a vertex id >= V");
+  if (outcome == gz::QueryOutcome::kTimeout) {
+    rc = fail(GZ_ERR_TIMEOUT, "a bounded device wait timed out");
   } else {
-    h->prof_acc.query_rounds += round + 1;
-    if (num_cc) *num_cc = ncc;
-    if (parent_out) std::copy(t.labels, t.labels + h->V, parent_out);
+    boruvka_account(h->tq.graph, t.pin, t.graph);
+    if (rounds) *rounds = round;
+    if (outcome == gz::QueryOutcome::kOutOfSamples) {
+      rc = fail(GZ_ERR_OUT_OF_SAMPLES, out_of_samples_msg(h, round));
+    } else if (outcome == gz::QueryOutcome::kBadSample) {
+      rc = fail(GZ_ERR_BAD_SAMPLE, "a sampled edge decoded to a vertex id >= V");
+    } else {
+      h->prof_acc.query_rounds += round + 1;
+      if (num_cc) *num_cc = ncc;
+      if (parent_out) std::copy(t.labels, t.labels + h->V, parent_out);
+    }
   }
   h->tq.pool.push_back(t);
   return rc;

@@ -565,21 +565,24 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
   return v;
 }
 
-// Barrier over every block of the launch. CL: the launch is one cluster (hardware barrier; threads
-// that have exited are not waited for). Otherwise the blocks of a cooperative launch count their
-// arrivals in *count (zeroed before the launch); barrier number k completes at k * gridDim.x
-// arrivals. Writes before it are seen by every block after it (release at the arrival, acquire
-// after it). A block with a failed warp (failed = true in any thread) leaves without arriving; a
-// block that waits longer than kWaitLimitNs sets the timeout status. Both return false, and the
-// caller returns from the kernel (the other blocks then time out at their next barrier).
+// Barrier over every block of the launch. CL: the launch is one cluster (hardware barrier). Otherwise
+// the blocks of a cooperative launch count their arrivals in *count (zeroed before the launch); barrier
+// number k completes at k * gridDim.x arrivals. Writes before it are seen by every block after it
+// (release at the arrival, acquire after it). False, and the caller returns from the kernel: for a
+// block with a failed warp (failed = true in any thread; it has set the timeout status) and for a block
+// that waits longer than kWaitLimitNs, which sets that status. The other blocks of a cooperative launch
+// then time out at their next barrier. Those of a cluster run on without the block, since threads that
+// have exited count as arrived; the failed block passes this barrier before it leaves, so that its status
+// bit is released to them, and a kernel that ends looks at the bit before it calls its work complete.
 template <bool CL>
 __device__ bool launch_barrier(uint32_t *count, uint32_t k, bool failed, uint32_t *status) {
-  if (__syncthreads_or(failed)) return false;
+  const bool left = __syncthreads_or(failed);
   if (CL) {
     __threadfence();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    return true;
+    return !left;
   }
+  if (left) return false;
   __shared__ uint32_t s_ok;
   if (threadIdx.x == 0) {
     __threadfence();

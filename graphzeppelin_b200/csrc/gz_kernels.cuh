@@ -4,14 +4,9 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
-namespace gz {
+#include "gz_status.h"
 
-// Status bits a kernel may raise in the handle's device status word.
-enum : uint32_t {
-  kStatusBadVertex = 1u << 0,
-  kStatusTimeout = 1u << 1,
-  kStatusBadSample = 1u << 2,
-};
+namespace gz {
 
 enum GutterInput : int {
   kInputRecords = 0,  // packed 9-byte records {u8 type, u32 src, u32 dst}: 2 endpoint entries

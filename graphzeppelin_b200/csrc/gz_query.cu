@@ -237,7 +237,8 @@ k_bv_query(BoruvkaGeom g, const uint32_t *__restrict__ sk_words, BoruvkaBufs b, 
         b.ctl[1] = modified ? 1u : 0u;
         b.ctl[2] = 0;
         *b.round = round;
-        *b.racc_dirty = 0;  // every accumulator was cleared by the root that read it
+        // every accumulator was cleared by the root that read it, unless a block gave up on the way
+        if (!(__ldcg(b.status) & kStatusTimeout)) *b.racc_dirty = 0;
       }
       break;
     }

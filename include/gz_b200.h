@@ -201,7 +201,8 @@ GZ_API int gz_has_cached_query(const gz_alg_t *alg, int query_code, int *out);
  * queued behind the query, so the caller never waits for it and the answer is the state at
  * submission without a copy of the sketches (queries interleaved with ingest). Several tickets
  * may be in flight. gz_query_wait blocks until its query is done and returns parent_out (NULL or
- * V entries), the component count and the rounds, or GZ_ERR_OUT_OF_SAMPLES / GZ_ERR_BAD_SAMPLE.
+ * V entries), the component count and the rounds, or GZ_ERR_OUT_OF_SAMPLES / GZ_ERR_BAD_SAMPLE /
+ * GZ_ERR_TIMEOUT (a device wait of the query, or of an update before it, gave up: nothing is written).
  * Device errors of earlier updates are reported by the next flush. Ticket queries leave the
  * handle's cached answer and update lock alone. */
 GZ_API int gz_query_submit(gz_alg_t *alg, uint64_t *ticket);
