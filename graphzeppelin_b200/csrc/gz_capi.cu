@@ -177,6 +177,8 @@ struct gz_alg {
   gz::BoruvkaBufs bv{};
   bool bv_alloc = false;
   uint32_t *d_final = nullptr, *d_ncc = nullptr;
+  uint2 *d_edges = nullptr;  // the spanning forest's edges, on their way to the host
+  uint32_t n_forest = 0;     // edges of the device answer's forest: one per union, V less its components
   bool dsu_valid = true, update_locked = false, labels_on_host = false;
   // eager DSU (the reference's default build, src/cc_sketch_alg.cpp:87-102): a host union-find
   // and the spanning-forest edge set, kept while dsu_valid; host_answer = it holds merges the
@@ -592,6 +594,7 @@ void destroy_alg(gz_alg *h) {
   }
   dev_free(h->d_raw);
   free_bv(h->bv);
+  dev_free(h->d_edges);
   for (auto &e : h->prof_pending) {
     cudaEventDestroy(e.a);
     cudaEventDestroy(e.b);
@@ -855,23 +858,31 @@ void pre_insert_one(gz_alg *h, uint32_t u, uint32_t v) {
   }
 }
 
+// The spanning forest of the last device answer: the count, and up to cap (src, dst) pairs into
+// edges_out (host memory; null: the count only).
+int forest_to_host(gz_alg *h, uint32_t *edges_out, size_t cap, size_t *n_edges) {
+  *n_edges = h->n_forest;
+  const size_t n = std::min<size_t>(cap, h->n_forest);
+  if (!edges_out || !n) return GZ_OK;
+  GZ_TRY(dev_alloc(&h->d_edges, h->V));
+  GZ_CUDA(gz::forest_edges(h->bv, h->V, h->d_edges, h->stream));
+  GZ_CUDA(cudaMemcpyAsync(edges_out, h->d_edges, n * sizeof(uint2), cudaMemcpyDeviceToHost, h->stream));
+  GZ_CUDA(cudaStreamSynchronize(h->stream));
+  return GZ_OK;
+}
+
 // Seed the eager DSU from the device answer (labels and Boruvka's spanning forest).
 int eager_from_device(gz_alg *h, bool have_forest) {
   h->hdsu.resize(h->V);
   GZ_CUDA(cudaMemcpyAsync(h->hdsu.data(), h->d_final, sizeof(uint32_t) * h->V, cudaMemcpyDeviceToHost, h->stream));
-  uint32_t n = 0;
-  std::vector<uint64_t> idx;
+  h->hforest.clear();
   if (have_forest) {
-    GZ_CUDA(cudaMemcpyAsync(h->h_status + 3, h->bv.forest_n, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    GZ_CUDA(cudaStreamSynchronize(h->stream));
-    n = std::min<uint32_t>(h->h_status[3], h->V);
-    idx.resize(n);
-    if (n) GZ_CUDA(cudaMemcpyAsync(idx.data(), h->bv.forest, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
+    std::vector<uint32_t> edges(2 * (size_t)h->V);
+    size_t n = 0;
+    GZ_TRY(forest_to_host(h, edges.data(), h->V, &n));
+    for (size_t i = 0; i < n; ++i) h->hforest.insert(((uint64_t)edges[2 * i] << 32) | edges[2 * i + 1]);
   }
   GZ_CUDA(cudaStreamSynchronize(h->stream));
-  idx.erase(std::remove(idx.begin(), idx.end(), gz::kNoEdge), idx.end());
-  h->hforest.clear();
-  h->hforest.insert(idx.begin(), idx.end());
   h->host_answer = false;
   return GZ_OK;
 }
@@ -909,13 +920,14 @@ int alloc_bv(gz::BoruvkaBufs &b, size_t V, uint32_t *status, uint32_t **labels, 
   k.take(&b.minv, V);
   k.take(&b.forest, V);
   k.take(labels, V);
-  k.take(&b.round, 8);  // round, ctl[3], components
+  k.take(&b.round, 8);  // round, ctl[3], components, forest edges
   k.take(&b.flags, 4);
   k.take(&b.forest_n, 1);
   k.take(&b.trace_n, 1);
   GZ_TRY(k.alloc(&b.block));
   b.ctl = b.round + 1;
   *ncc = b.round + 4;
+  b.edge_n = b.round + 5;
   b.status = status;
   return GZ_OK;
 }
@@ -1080,6 +1092,7 @@ int run_boruvka(gz_alg *h) {
   h->prof_acc.query_rounds += round + 1;
   GZ_TRY(status_result(h));
   h->last_ncc = h->h_qpin[2];
+  h->n_forest = h->V - h->last_ncc;
   h->last_rounds = round;
   h->dsu_valid = true;
   h->labels_on_host = false;
@@ -1117,6 +1130,7 @@ int ensure_answer(gz_alg *h) {
     GZ_CUDA(cudaMemcpyAsync(h->h_status + 2, h->d_ncc, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     GZ_CUDA(cudaStreamSynchronize(h->stream));
     h->last_ncc = h->h_status[2];
+    h->n_forest = 0;
     return GZ_OK;
   }
   h->query_running = true;
@@ -1599,21 +1613,7 @@ int gz_spanning_forest(gz_alg_t *h, uint32_t *edges_out, size_t cap, size_t *n_e
     }
     return GZ_OK;
   }
-  uint32_t n = 0;
-  GZ_CUDA(cudaMemcpyAsync(h->h_status + 3, h->bv.forest_n, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-  GZ_CUDA(cudaStreamSynchronize(h->stream));
-  n = std::min<uint32_t>(h->h_status[3], h->V);
-  std::vector<uint64_t> idx(n);
-  if (n) GZ_CUDA(cudaMemcpy(idx.data(), h->bv.forest, n * sizeof(uint64_t), cudaMemcpyDeviceToHost));
-  idx.erase(std::remove(idx.begin(), idx.end(), gz::kNoEdge), idx.end());
-  *n_edges = idx.size();
-  if (edges_out) {
-    for (size_t i = 0; i < std::min(cap, idx.size()); ++i) {
-      edges_out[2 * i] = (uint32_t)(idx[i] >> 32);
-      edges_out[2 * i + 1] = (uint32_t)idx[i];
-    }
-  }
-  return GZ_OK;
+  return forest_to_host(h, edges_out, cap, n_edges);
 }
 
 int gz_dump_sketches(gz_alg_t *h, void *buf, size_t bytes) {

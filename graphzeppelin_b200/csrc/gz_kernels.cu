@@ -1299,6 +1299,29 @@ __global__ void k_bv_final(uint32_t V, uint32_t *parent, uint32_t *out, uint32_t
   if (v < V) bv_final_vertex(v, parent, out, ncc);
 }
 
+// The one-launch query leaves a place per vertex, empty or holding the edge that linked it: a host copy
+// of the places moved 8 V bytes and picked the edges out there, also to count them (2^20 vertices: 2.5 ms
+// to count, 11.4 to count and fetch). With this kernel the fetch moves the edges alone (1.3 ms).
+__global__ void __launch_bounds__(1024)
+k_forest_edges(const uint64_t *__restrict__ forest, const uint32_t *__restrict__ forest_n, uint32_t V,
+               uint2 *__restrict__ out, uint32_t *__restrict__ count) {
+  __shared__ uint32_t s_warp[32], s_base;
+  const uint32_t i = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t idx = i < min(*forest_n, V) ? forest[i] : kNoEdge;
+  const uint32_t m = __ballot_sync(kFull, idx != kNoEdge);
+  if (lane == 0) s_warp[warp] = __popc(m);
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+  for (uint32_t w = 0; w < 32; ++w) {
+    before += w < warp ? s_warp[w] : 0u;
+    total += s_warp[w];
+  }
+  if (threadIdx.x == 0) s_base = total ? atomicAdd(count, total) : 0u;
+  __syncthreads();
+  if (idx != kNoEdge)
+    out[s_base + before + __popc(m & ((1u << lane) - 1u))] = make_uint2((uint32_t)(idx >> 32), (uint32_t)idx);
+}
+
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -1561,6 +1584,14 @@ cudaError_t boruvka_reset(const BoruvkaGeom &g, const BoruvkaBufs &b, cudaStream
   g_launches++;
   cudaMemsetAsync(b.forest_n, 0, sizeof(uint32_t), s);
   if (b.trace) cudaMemsetAsync(b.trace_n, 0, sizeof(uint32_t), s);
+  return cudaGetLastError();
+}
+
+cudaError_t forest_edges(const BoruvkaBufs &b, uint32_t V, uint2 *out, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(b.edge_n, 0, sizeof(uint32_t), s);
+  if (e != cudaSuccess) return e;
+  k_forest_edges<<<blocks_for(V, 1024), 1024, 0, s>>>(b.forest, b.forest_n, V, out, b.edge_n);
+  g_launches++;
   return cudaGetLastError();
 }
 

@@ -240,6 +240,7 @@ struct BoruvkaBufs {
   uint32_t *racc_dirty;  // 1   racc may hold leftovers (first use; a query that did not finish)
   uint64_t *forest;      // V   spanning-forest edge indices (entries of kNoEdge are empty)
   uint32_t *forest_n;    // 1   entries in use, empty ones included
+  uint32_t *edge_n;      // 1   forest_edges' places handed out
   void *trace;           // gz_trace_rec_t[trace_cap] or null
   uint32_t *trace_n;     // 1
   uint32_t trace_cap;
@@ -272,6 +273,9 @@ cudaError_t sketch_total_xor(const uint8_t *sketches, uint32_t V, uint32_t sketc
                              uint32_t *total, cudaStream_t s);
 
 cudaError_t boruvka_reset(const BoruvkaGeom &g, const BoruvkaBufs &b, cudaStream_t s);
+// The edges of the last query's spanning forest written to out[0 ..) (V - 1 at most) as {smaller,
+// larger} vertex id, in no particular order.
+cudaError_t forest_edges(const BoruvkaBufs &b, uint32_t V, uint2 *out, cudaStream_t s);
 cudaError_t boruvka_round0(const BoruvkaGeom &g, const uint8_t *sketches, const BoruvkaBufs &b,
                            cudaStream_t s);
 // one round >= 1; the round number is read from b.round
