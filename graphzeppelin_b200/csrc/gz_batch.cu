@@ -26,6 +26,7 @@
 #include "gz_device.cuh"
 #include "gz_kernels.cuh"
 #include "gz_planes.cuh"
+#include "gz_ingest_plan.h"
 
 void gz_internal_set_error(const std::string &msg);
 
@@ -1647,6 +1648,7 @@ struct gz_batch {
   // gutter
   uint2 *d_entries = nullptr;
   uint64_t entry_cap = 0;
+  gz::FailedSize no_coded;  // entries of a buffer for coded entries that could not be had
   uint64_t *d_bins = nullptr, *d_scan_tmp = nullptr, *d_total = nullptr;
   uint32_t *d_bin_fill = nullptr;  // per-bin slots taken by the sort-scatter pass
   uint32_t *d_bin_off = nullptr;
@@ -1665,6 +1667,7 @@ struct gz_batch {
   // one-launch query: accumulators; states and deterministic buckets (6 words a vertex); the results
   // (ncc, lastmod) and control words, and the results on the host
   uint32_t *d_racc = nullptr, *d_vstate = nullptr, *d_qres = nullptr, *h_qres = nullptr;
+  gz::FailedSize no_launch;  // vertices whose buffers could not be had
   bool racc_dirty = true;  // d_racc may hold nonzero words
   uint64_t cap_racc = 0, cap_vstate = 0, cap_qres = 0, cap_hqres = 0;
   uint32_t *d_order = nullptr, *d_order_comp = nullptr, *d_comp_start = nullptr, *d_ncomp = nullptr, *d_acc = nullptr;
@@ -1982,8 +1985,10 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
       if (off[g + 1] > off[g] && !route_sparse(h, gd, off[g + 1] - off[g]))
         coded = gd.plane && coded_entry_fits(gd.V, gd.C, gd.bin_shift);
     }
+    coded = coded && (h->entry_cap >= 4 * n_dense || h->no_coded.may_try(4 * n_dense));
     if (coded && grow(&h->d_entries, h->entry_cap, 4 * n_dense, h->stream) != GZ_OK) {
       cudaGetLastError();
+      h->no_coded.failed(4 * n_dense);
       coded = false;
     }
     if (!coded) MB_TRY(grow(&h->d_entries, h->entry_cap, 2 * n_dense, h->stream));
@@ -2172,7 +2177,7 @@ constexpr uint64_t kMbOneLaunchMaxV = 1u << 23;
 constexpr uint32_t kQresCtl = 8;  // go, barrier
 bool one_launch_buffers(gz_batch *h) {
   const uint64_t V = h->total_V;
-  if (V > kMbOneLaunchMaxV) return false;
+  if (V > kMbOneLaunchMaxV || !h->no_launch.may_try(V)) return false;
   int rc = ensure_parent(h);
   const uint64_t had = h->d_racc ? h->cap_racc : 0;
   if (rc == GZ_OK) rc = grow(&h->d_racc, h->cap_racc, V * racc_words(1, h->max_B), h->stream);
@@ -2189,6 +2194,7 @@ bool one_launch_buffers(gz_batch *h) {
   }
   if (rc == GZ_OK) return true;
   cudaGetLastError();
+  h->no_launch.failed(V);
   mb_free(h->d_racc);
   mb_free(h->d_vstate);
   h->cap_racc = h->cap_vstate = 0;

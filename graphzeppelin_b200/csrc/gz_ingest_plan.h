@@ -1,6 +1,7 @@
 // Plans of record ingest, host-only C++ shared by the library and its CPU unit tests: how a host
 // call's records are cut into host->device copies and when the gutter is folded into the sketches
-// (IngestPlan), and which calls go straight to the sketches instead of the gutter (DirectRoute).
+// (IngestPlan), which calls go straight to the sketches instead of the gutter (DirectRoute), and which
+// optional buffers are not asked for again (FailedSize).
 //
 // The copies run on a second stream into kStageBuffers device buffers while the gutter and the
 // sketch update run on the handle's stream. A long call is cut so that the sketch update overlaps
@@ -109,6 +110,15 @@ struct DirectRoute {
     return true;
   }
   void flushed() { sent = 0; }
+};
+
+// Sizes at which an optional buffer could not be had. The caller then takes the form that does without, and
+// does not ask for as much again: a failed allocation costs milliseconds, and a growing buffer gives
+// its old block up first.
+struct FailedSize {
+  uint64_t least = ~0ull;
+  bool may_try(uint64_t size) const { return size < least; }
+  void failed(uint64_t size) { least = std::min(least, size); }
 };
 
 }  // namespace gz
