@@ -1664,12 +1664,14 @@ struct gz_batch {
   uint64_t *d_res = nullptr;
   uint32_t *d_res_g = nullptr;
   uint64_t cap_res = 0, cap_res_g = 0;
-  // one-launch query: accumulators; states and deterministic buckets (6 words a vertex); the results
-  // (ncc, lastmod) and control words, and the results on the host
-  uint32_t *d_racc = nullptr, *d_vstate = nullptr, *d_qres = nullptr, *h_qres = nullptr;
-  gz::FailedSize no_launch;  // vertices whose buffers could not be had
-  bool racc_dirty = true;  // d_racc may hold nonzero words
-  uint64_t cap_racc = 0, cap_vstate = 0, cap_qres = 0, cap_hqres = 0;
+  // one-launch query: accumulators from the start of one block, states and deterministic buckets (6 words a
+  // vertex) at its end; the results (ncc, lastmod) and control words, and the results on the host
+  uint32_t *d_qbuf = nullptr, *d_qres = nullptr, *h_qres = nullptr;
+  bool qbuf_plain = false;      // d_qbuf came from cudaMalloc, not from the stream-ordered pool
+  uint32_t *racc = nullptr;     // block of the last query: d_qbuf, or d_entries
+  uint64_t racc_zero = 0;       // words from its start known to be zero
+  gz::FailedSize no_launch;     // vertices whose buffers could not be had
+  uint64_t cap_qbuf = 0, cap_qres = 0, cap_hqres = 0;
   uint32_t *d_order = nullptr, *d_order_comp = nullptr, *d_comp_start = nullptr, *d_ncomp = nullptr, *d_acc = nullptr;
   uint32_t *d_active = nullptr, *d_modified = nullptr, *d_round = nullptr, *d_ncc = nullptr;
   cudaGraphExec_t round_exec = nullptr;
@@ -1761,8 +1763,7 @@ void batch_destroy(gz_batch *h) {
   mb_free(h->d_modified);
   mb_free(h->d_round);
   mb_free(h->d_ncc);
-  mb_free(h->d_racc);
-  mb_free(h->d_vstate);
+  mb_free(h->d_qbuf);
   mb_free(h->d_qres);
   if (h->h_qres) cudaFreeHost(h->h_qres);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -1985,6 +1986,7 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
       if (off[g + 1] > off[g] && !route_sparse(h, gd, off[g + 1] - off[g]))
         coded = gd.plane && coded_entry_fits(gd.V, gd.C, gd.bin_shift);
     }
+    if (h->racc == reinterpret_cast<uint32_t *>(h->d_entries)) h->racc_zero = 0;  // entries take its place
     coded = coded && (h->entry_cap >= 4 * n_dense || h->no_coded.may_try(4 * n_dense));
     if (coded && grow(&h->d_entries, h->entry_cap, 4 * n_dense, h->stream) != GZ_OK) {
       cudaGetLastError();
@@ -2169,20 +2171,47 @@ int enqueue_round(gz_batch *h, cudaStream_t s) {
 }
 
 // Buffers of the one-launch query. False: they do not fit, or the vertices are more than 2^23; the rounds of
-// batch_query_rounds then run. The line bounds the accumulators (about 350 to 500 B a vertex, 4 GB) and
-// their one allocation (a handle's first query of 8.2e6 vertices takes 22 ms against 18 in rounds). Graphs
-// of 1024 vertices, launch against rounds: 1.02e6 vertices together 1.5 and 2.5 ms, 2.05e6 2.8 and 4.3,
-// 4.1e6 5.4 and 7.7, 8.2e6 10.8 and 14.7.
+// batch_query_rounds then run. Graphs of 1024 vertices, launch against rounds: 1.02e6 vertices together 1.5
+// and 2.5 ms, 2.05e6 2.8 and 4.3, 4.1e6 5.4 and 7.7, 8.2e6 10.8 and 14.7.
+// The accumulators take about 350 to 500 B a vertex. Where the gutter's entry buffer, idle between
+// ingests, is large enough they lie there, and are cleared by the first query after an ingest. Otherwise the
+// handle's first block comes from cudaMalloc when it is large: the stream-ordered pool grew by 512 MB in 3.2
+// ms and by 2 GB in 12 to 51, cudaMalloc gives them in 0.6 to 1.7 and 0.7 to 3.5. A block that is outgrown goes
+// on from the pool, whose regrowth does not wait for the device. (A process's first query, graphs of 1024
+// vertices with 6,000 records each: 2.05e6 vertices 7.6 -> 4.6 ms, 8.2e6 27 -> 13.3, with 600 records each 28
+// -> 14; in rounds 5.7, 16.7 and 17.4.)
 constexpr uint64_t kMbOneLaunchMaxV = 1u << 23;
 constexpr uint32_t kQresCtl = 8;  // go, barrier
+constexpr uint64_t kQbufPlainWords = 1ull << 24;  // 64 MB
+uint64_t racc_total_words(const gz_batch *h) { return h->total_V * racc_words(1, h->max_B); }
+// where the states start in a block of cap words
+uint64_t vstate_at(const gz_batch *h, uint64_t cap) { return (cap - (6 * h->total_V + 4)) & ~63ull; }
+int grow_qbuf(gz_batch *h, uint64_t words) {
+  if (h->d_qbuf && h->cap_qbuf >= words) return GZ_OK;
+  const uint64_t n = headroom(h->cap_qbuf, words);
+  const bool plain = !h->d_qbuf && n >= kQbufPlainWords;
+  h->cap_qbuf = h->racc_zero = 0;
+  if (h->qbuf_plain) mb_free(h->d_qbuf);
+  h->qbuf_plain = false;
+  if (plain) MB_TRY(mb_alloc(&h->d_qbuf, n));
+  else MB_TRY(mb_realloc_async(&h->d_qbuf, n, h->stream));
+  h->qbuf_plain = plain;
+  h->cap_qbuf = n;
+  return GZ_OK;
+}
 bool one_launch_buffers(gz_batch *h) {
   const uint64_t V = h->total_V;
   if (V > kMbOneLaunchMaxV || !h->no_launch.may_try(V)) return false;
   int rc = ensure_parent(h);
-  const uint64_t had = h->d_racc ? h->cap_racc : 0;
-  if (rc == GZ_OK) rc = grow(&h->d_racc, h->cap_racc, V * racc_words(1, h->max_B), h->stream);
-  if (h->cap_racc != had) h->racc_dirty = true;
-  if (rc == GZ_OK) rc = grow(&h->d_vstate, h->cap_vstate, 6 * V + 4, h->stream);
+  const uint64_t words = racc_total_words(h) + 6 * V + 4 + 64;
+  const bool own = h->d_qbuf && h->cap_qbuf >= words;
+  uint32_t *racc = reinterpret_cast<uint32_t *>(h->d_entries);
+  if (own || !racc || 2 * h->entry_cap < words) {
+    if (rc == GZ_OK) rc = grow_qbuf(h, words);
+    racc = h->d_qbuf;
+  }
+  if (h->racc != racc) h->racc_zero = 0;
+  h->racc = racc;
   if (rc == GZ_OK) rc = grow(&h->d_qres, h->cap_qres, 2 * (uint64_t)h->G + kQresCtl, h->stream);
   if (rc == GZ_OK && (!h->h_qres || h->cap_hqres < 2 * (uint64_t)h->G)) {
     const uint64_t n = headroom(h->cap_hqres, 2 * (uint64_t)h->G);
@@ -2195,20 +2224,24 @@ bool one_launch_buffers(gz_batch *h) {
   if (rc == GZ_OK) return true;
   cudaGetLastError();
   h->no_launch.failed(V);
-  mb_free(h->d_racc);
-  mb_free(h->d_vstate);
-  h->cap_racc = h->cap_vstate = 0;
+  mb_free(h->d_qbuf);
+  h->qbuf_plain = false;
+  h->racc = nullptr;
+  h->cap_qbuf = h->racc_zero = 0;
   return false;
 }
 
-// One cooperative launch for every round of every graph, one synchronisation.
-int batch_query_launch(gz_batch *h, uint32_t *labels_out) {
+// One cooperative launch for every round of every graph, one synchronisation. *zero_after: racc_zero once it
+// has run to its end.
+int batch_query_launch(gz_batch *h, uint32_t *labels_out, uint64_t *zero_after) {
   const MBBufs b = h->bufs();
   const uint32_t V = (uint32_t)h->total_V, G = h->G;
   MbQuery q{};
-  q.rstate = h->d_vstate;
-  q.det = h->d_vstate + 2 * (((uint64_t)V + 1) & ~1ull);
-  q.racc = h->d_racc;
+  const uint64_t racc_total = racc_total_words(h);
+  const uint64_t states = vstate_at(h, h->racc == h->d_qbuf ? h->cap_qbuf : 2 * h->entry_cap);
+  q.racc = h->racc;
+  q.rstate = h->racc + states;
+  q.det = q.rstate + 2 * (((uint64_t)V + 1) & ~1ull);
   q.go = h->d_qres;
   q.qbar = q.go + 1;
   q.ncc = h->d_qres + kQresCtl;
@@ -2231,8 +2264,11 @@ int batch_query_launch(gz_batch *h, uint32_t *labels_out) {
   const int blocks = std::min<int>(num_sms(), (int)cdiv(nbatch, warps));
   MB_CUDA(cudaMemsetAsync(q.qbar, 0, sizeof(uint32_t), h->stream));
   // a query that ran to its end leaves every accumulator zero
-  if (h->racc_dirty) MB_CUDA(cudaMemsetAsync(h->d_racc, 0, sizeof(uint32_t) * h->cap_racc, h->stream));
-  h->racc_dirty = true;
+  const uint64_t zero = h->racc_zero;
+  h->racc_zero = 0;
+  if (zero < racc_total)
+    MB_CUDA(cudaMemsetAsync(h->racc + zero, 0, sizeof(uint32_t) * (racc_total - zero), h->stream));
+  *zero_after = std::min(std::max(zero, racc_total), states);
   MBBufs a_b = b;
   void *args[] = {&a_b, &q};
   MB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(blocks), dim3(32 * warps), args,
@@ -2256,7 +2292,8 @@ int batch_query(gz_batch *h, uint32_t *labels_out) {
     cudaEventCreate(&q1);
     cudaEventRecord(q0, h->stream);
   }
-  int rc = batch_query_launch(h, labels_out);
+  uint64_t zero_after = 0;
+  int rc = batch_query_launch(h, labels_out, &zero_after);
   if (h->prof) cudaEventRecord(q1, h->stream);
   const int rc_flush = batch_flush_status(h);
   if (rc == GZ_OK) rc = rc_flush;
@@ -2267,7 +2304,7 @@ int batch_query(gz_batch *h, uint32_t *labels_out) {
     cudaEventDestroy(q1);
   }
   if (rc == GZ_OK || rc == GZ_ERR_BAD_SAMPLE) {
-    h->racc_dirty = false;
+    h->racc_zero = zero_after;
     h->ncc.assign(h->h_qres, h->h_qres + G);
     h->rounds.assign(h->h_qres + G, h->h_qres + 2 * (size_t)G);
     h->status.assign(G, GZ_OK);
