@@ -260,33 +260,39 @@ __global__ void k_mb_bin_off(const uint64_t *scanned, uint64_t nbins, const uint
 // For a graph whose call brings too few records to pay for the gutter and its tiles, each record is
 // hashed once by a warp, a lane per column, and XORed into both endpoints' sketches in HBM with
 // global reductions (warp_record_global: bound by L2's rate for them, about 45e9 sectors/s). A
-// self-loop XORs one sketch twice: no change, as in the gutter path. The warps of the grid take runs
-// of 32 records of the record tiles (32 lanes read them at once). (Sketches of more than 31 columns,
-// k_mb_direct_wide: a thread per record.)
-__global__ void __launch_bounds__(256)
+// self-loop XORs one sketch twice: no change, as in the gutter path. A block takes a record tile, or one
+// of `pieces` interleaved parts of each where there are few tiles, and deals its records evenly to the
+// warps that work on the tile, at most 32 at a time (the lanes read them at once): a tile of a small
+// graph is not one warp's. (Sketches of more than 31 columns, k_mb_direct_wide: a thread per record.)
+constexpr uint32_t kMbDirectThreads = 256;
+constexpr uint32_t kMbDirectPieces = kMbRecTile / kMbDirectThreads;  // at most: 32 records a warp then
+__global__ void __launch_bounds__(kMbDirectThreads)
 k_mb_direct(const uint8_t *__restrict__ rec, uint64_t n_rec, const uint4 *__restrict__ rtiles, uint32_t n_rt,
-            const GraphDesc *__restrict__ graphs, uint8_t *__restrict__ sketches,
+            uint32_t pieces, const GraphDesc *__restrict__ graphs, uint8_t *__restrict__ sketches,
             const uint64_t *__restrict__ flip, uint32_t *__restrict__ status) {
-  constexpr uint32_t kRuns = kMbRecTile / 32;
-  const uint32_t lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rt * kRuns; r += nwarps) {
-    const uint4 rt = rtiles[r / kRuns];
-    const uint32_t i0 = (r % kRuns) * 32;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = pieces * (kMbDirectThreads / 32);
+  for (uint32_t item = blockIdx.x; item < n_rt * pieces; item += gridDim.x) {
+    const uint4 rt = rtiles[item / pieces];
+    const uint32_t per = min((rt.w + nwarps - 1) / nwarps, 32u);  // records a warp takes at once
+    uint32_t i0 = (item % pieces * (kMbDirectThreads / 32) + warp) * per;
     if (i0 >= rt.w) continue;
     const GraphDesc gd = graphs[rt.x];
     const uint64_t kc = xxh3_premix(flip[gd.flip_off + min(lane, gd.C)]);
     const uint64_t kchk = xxh3_premix(flip[gd.flip_off + gd.C]);
     uint32_t *gsk = reinterpret_cast<uint32_t *>(sketches + gd.sk_off);
-    uint32_t mu = 0, mv = 0;
-    if (i0 + lane < rt.w) load_record(rec, rec + 9 * n_rec, (((uint64_t)rt.z << 32) | rt.y) + i0 + lane, mu, mv);
-    if (mu >= gd.V || mv >= gd.V) {
-      atomicOr(status, kStatusBadVertex);
-      mu = mv;  // dropped
-    }
-    for (uint32_t m = __ballot_sync(kFull, mu != mv); m; m &= m - 1) {
-      const uint32_t u = __shfl_sync(kFull, mu, __ffs(m) - 1), v = __shfl_sync(kFull, mv, __ffs(m) - 1);
-      warp_record_global(gsk + (uint64_t)u * gd.sketch_words, gsk + (uint64_t)v * gd.sketch_words, u, v, gd.C, gd.B,
-                         kc, kchk);
+    for (; i0 < rt.w; i0 += nwarps * per) {
+      uint32_t mu = 0, mv = 0;
+      if (lane < per && i0 + lane < rt.w)
+        load_record(rec, rec + 9 * n_rec, (((uint64_t)rt.z << 32) | rt.y) + i0 + lane, mu, mv);
+      if (mu >= gd.V || mv >= gd.V) {
+        atomicOr(status, kStatusBadVertex);
+        mu = mv;  // dropped
+      }
+      for (uint32_t m = __ballot_sync(kFull, mu != mv); m; m &= m - 1) {
+        const uint32_t u = __shfl_sync(kFull, mu, __ffs(m) - 1), v = __shfl_sync(kFull, mv, __ffs(m) - 1);
+        warp_record_global(gsk + (uint64_t)u * gd.sketch_words, gsk + (uint64_t)v * gd.sketch_words, u, v, gd.C, gd.B,
+                           kc, kchk);
+      }
     }
   }
 }
@@ -1950,7 +1956,7 @@ bool route_sparse(const gz_batch *h, const GraphDesc &gd, uint64_t n) {
 // records of graph g are d_rec[off[g] .. off[g+1]) (9-byte records)
 int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
   std::vector<uint4> rt_dense, rt_sparse;
-  uint64_t n_dense = 0;
+  uint64_t n_dense = 0, n_sparse = 0;
   for (uint32_t g = 0; g < h->G; ++g) {
     if (off[g + 1] < off[g]) return mb_fail(GZ_ERR_INVALID, "record offsets must be non-decreasing");
     const uint64_t n = off[g + 1] - off[g];
@@ -1961,7 +1967,7 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
       const uint32_t cnt = (uint32_t)std::min<uint64_t>(kMbRecTile, off[g + 1] - s);
       rt.push_back(make_uint4(g, (uint32_t)s, (uint32_t)(s >> 32), cnt));
     }
-    if (!sparse) n_dense += n;
+    (sparse ? n_sparse : n_dense) += n;
   }
   if (rt_dense.empty() && rt_sparse.empty()) return GZ_OK;
   if (2 * n_dense >= 0xFFFFFFF0ull) return mb_fail(GZ_ERR_INVALID, "more than 2^31 records in one batch ingest");
@@ -2070,9 +2076,13 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
   }
   if (!rt_sparse.empty()) {
     if (h->max_C <= kPlaneMaxColumns) {
-      const uint64_t warps = rt_sparse.size() * (kMbRecTile / 32);
-      const unsigned grid = (unsigned)std::min<uint64_t>((warps + 7) / 8, (uint64_t)num_sms() * 8);
-      k_mb_direct<<<grid, 256, 0, h->stream>>>(rec, off[h->G], h->d_rtiles + n_rt_dense, (uint32_t)rt_sparse.size(),
+      // parts of a tile: 32 records a warp in an average one, and enough parts for the whole GPU
+      const uint32_t n_rt_sparse = (uint32_t)rt_sparse.size(), resident = (uint32_t)num_sms() * 8;
+      const uint32_t average = cdiv(n_sparse, n_rt_sparse);
+      const uint32_t pieces = std::min(kMbDirectPieces, std::max(cdiv(average, kMbDirectThreads),
+                                                                 cdiv(2 * resident, n_rt_sparse)));
+      const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)n_rt_sparse * pieces, resident);
+      k_mb_direct<<<grid, kMbDirectThreads, 0, h->stream>>>(rec, off[h->G], h->d_rtiles + n_rt_dense, n_rt_sparse, pieces,
                                                h->d_graphs, h->d_sk, h->d_flip, h->d_status);
     } else {
       MB_CUDA(smem_optin(k_mb_direct_wide));
