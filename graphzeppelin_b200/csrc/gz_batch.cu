@@ -46,6 +46,7 @@ struct GraphDesc {
   uint32_t nbins, ntiles;
   uint32_t direct_max;  // staged form: tiles with fewer entries are updated in place in HBM
   uint32_t plane;       // its tiles are those of the bucket-plane form
+  uint32_t chosen;      // the form is the engine's choice (no tile size or CTA shape asked for)
 };
 
 // ---- gutter ----------------------------------------------------------------------------------
@@ -1837,6 +1838,8 @@ bool plane_fits(const GraphDesc &gd) {
   return gd.C <= kPlaneMaxColumns && gd.V <= (uint64_t)kMbBinsMax * kMbTilesPerBinMax << kMbPlaneShift;
 }
 
+constexpr uint32_t kMbStagedMaxV = 512;  // largest graph whose tiling choose_forms changes
+
 // Device bytes of one graph's sketches: V rounded up to 64 (any tile stays inside), 256-aligned.
 uint64_t graph_sketch_bytes(const GraphDesc &gd) {
   const uint64_t v_pad = ((uint64_t)gd.V + 63) & ~63ull;
@@ -1918,6 +1921,7 @@ int layout(gz_batch *h, const std::vector<uint32_t> &vpt_req) {
     // bucket planes unless a tile size or a CTA shape is asked for
     const bool plane = !vpt && h->threads == 1024 && h->ctas_per_sm == 1 && plane_fits(gd);
     MB_TRY(choose_tiles(gd, vpt, budget, plane));
+    gd.chosen = plane ? 1 : 0;
     gd.sk_off = sk_off;
     gd.flip_off = (uint32_t)flip_off;
     sk_off += graph_sketch_bytes(gd);
@@ -1941,27 +1945,87 @@ int batch_flush_status(gz_batch *h) {
   return GZ_OK;
 }
 
-// Whether graph gd takes n records of one call in place (sparse route). Bucket planes: a record in
-// place costs about 2 x 30 sector reductions (1.3 ns of the GPU at L2's 45e9 a second), a tile of 8
-// vertices with few entries about 25 ns: in place while the call brings fewer than about 4 entries a
-// vertex. Staged tiles: staging the touched tiles moves about 2 x V x sketch bytes over HBM plus the
-// gutter's bytes, in place takes about 2 (C + 1) bucket sectors of 64 B per record.
-bool route_sparse(const gz_batch *h, const GraphDesc &gd, uint64_t n) {
-  if (gd.plane) return 2.0 * (double)n < 4.0 * gd.V * h->sparse_factor;
+// Whether graph gd takes n records of one call in place (sparse route), call_bytes: the sketches of the
+// call's graphs. A form of the engine's choice: in place while the call brings fewer entries a vertex than
+//   36   sketches that lie in L2 (2e4 vertices, graphs of 64 / 4096: 16 entries 52 / 48 us in place, 91 / 85
+//        through planes, 32 92 / 80 and 100 / 92, 64 226 / 129 and 126 / 96);
+//   2.5  more than 1 GB, graphs past 128 vertices: a record in place is then 1.3 ns of L2 reductions, a vertex
+//        through planes 1.3 ns (1e6 vertices in graphs of 1024: 2 entries 1.29 ms in place, 3.9 2.29, any
+//        through planes about 1.33);
+//   4    otherwise (1.5e5 vertices in graphs of 1024: 3.9 entries 0.26 ms in place, 0.27 through planes).
+// Staged tiles asked for: staging the touched tiles moves about 2 x V x sketch bytes over HBM plus the gutter's
+// bytes, in place takes about 2 (C + 1) bucket sectors of 64 B per record.
+constexpr uint64_t kMbResidentBytes = 1ull << 27, kMbWideBytes = 1ull << 30;
+bool route_sparse(const gz_batch *h, const GraphDesc &gd, uint64_t n, uint64_t call_bytes) {
+  if (gd.chosen) {
+    const double line = call_bytes <= kMbResidentBytes ? 36.0 : call_bytes > kMbWideBytes && gd.V > 128 ? 2.5 : 4.0;
+    return 2.0 * (double)n < line * gd.V * h->sparse_factor;
+  }
   const double staged = 2.0 * gd.V * (gd.sketch_words * 4.0) + 50.0 * n;
   const double in_place = 128.0 * (gd.C + 1) * (double)n;
   return in_place < staged * h->sparse_factor;
+}
+
+// Sketch bytes of the graphs that bring records.
+uint64_t call_sketch_bytes(const gz_batch *h, const uint64_t *off) {
+  uint64_t bytes = 0;
+  for (size_t g = 0; g < h->graphs.size(); ++g)
+    if (off[g + 1] > off[g]) bytes += (uint64_t)h->graphs[g].V * h->graphs[g].sketch_words * 4;
+  return bytes;
+}
+
+// Form of a call's guttered graphs where the engine chooses it. Whole sketches of small graphs, staged 32 to a
+// tile, are moved for little, and their plain entries are scattered faster than coded ones: for calls that
+// bring few entries a vertex and no larger graph's (whose entries would have to be plain with theirs) the
+// small graphs are tiled for it. Staged against planes, ms: 1e6 vertices in graphs of 32, 8 entries a vertex
+// 1.76 and 2.37; of 64, 16 1.53 and 2.11, 64 3.30 and 3.28; of 256, 32 1.80 and 2.14, 64 3.02 and 2.98; of 512,
+// 16 1.89 and 1.74, 32 2.08 and 2.15; of 1024, 32 2.14 and 2.16. *changed: the tiling did.
+bool staged_suits(const GraphDesc &gd, uint64_t n) {
+  const double entries = 2.0 * (double)n / gd.V;
+  return gd.V <= 256 ? entries < 48 : gd.V <= kMbStagedMaxV && entries >= 24 && entries < 40;
+}
+int choose_forms(gz_batch *h, const uint64_t *off, uint64_t call_bytes, bool *changed) {
+  *changed = false;
+  bool any = false, staged = true;
+  for (size_t g = 0; g < h->graphs.size() && staged; ++g) {
+    const GraphDesc &gd = h->graphs[g];
+    const uint64_t n = off[g + 1] - off[g];
+    if (!n || route_sparse(h, gd, n, call_bytes)) continue;
+    any = true;
+    staged = gd.chosen && staged_suits(gd, n);
+  }
+  if (!any) return GZ_OK;  // nothing guttered: either tiling serves
+  size_t budget = 0;
+  for (GraphDesc &gd : h->graphs) {
+    const bool plane = !(staged && gd.V <= kMbStagedMaxV);
+    if (!gd.chosen || (gd.plane != 0) == plane) continue;
+    if (!budget) {
+      uint32_t max_C = 0;
+      for (const GraphDesc &x : h->graphs) max_C = std::max(max_C, x.C);
+      budget = tile_budget(h, max_C);
+    }
+    uint32_t vpt = 4;  // a tile no larger than the graph
+    while (vpt < 64 && vpt < gd.V && (uint64_t)gd.sketch_words * 4 * 2 * vpt <= budget) vpt *= 2;
+    MB_TRY(choose_tiles(gd, vpt, budget, plane));
+    *changed = true;
+  }
+  return GZ_OK;
 }
 
 // records of graph g are d_rec[off[g] .. off[g+1]) (9-byte records)
 int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
   std::vector<uint4> rt_dense, rt_sparse;
   uint64_t n_dense = 0, n_sparse = 0;
-  for (uint32_t g = 0; g < h->G; ++g) {
+  for (uint32_t g = 0; g < h->G; ++g)
     if (off[g + 1] < off[g]) return mb_fail(GZ_ERR_INVALID, "record offsets must be non-decreasing");
+  const uint64_t call_bytes = call_sketch_bytes(h, off);
+  bool retiled = false;
+  MB_TRY(choose_forms(h, off, call_bytes, &retiled));
+  if (retiled) MB_TRY(finalize_graphs(h));
+  for (uint32_t g = 0; g < h->G; ++g) {
     const uint64_t n = off[g + 1] - off[g];
     if (!n) continue;
-    const bool sparse = route_sparse(h, h->graphs[g], n);
+    const bool sparse = route_sparse(h, h->graphs[g], n, call_bytes);
     auto &rt = sparse ? rt_sparse : rt_dense;
     for (uint64_t s = off[g]; s < off[g + 1]; s += kMbRecTile) {
       const uint32_t cnt = (uint32_t)std::min<uint64_t>(kMbRecTile, off[g + 1] - s);
@@ -1989,7 +2053,7 @@ int batch_ingest(gz_batch *h, const void *d_rec, const uint64_t *off) {
     // coded entries (16 bytes) when every guttered graph's codes fit them, else plain ones (8)
     for (uint32_t g = 0; g < h->G && coded; ++g) {
       const GraphDesc &gd = h->graphs[g];
-      if (off[g + 1] > off[g] && !route_sparse(h, gd, off[g + 1] - off[g]))
+      if (off[g + 1] > off[g] && !route_sparse(h, gd, off[g + 1] - off[g], call_bytes))
         coded = gd.plane && coded_entry_fits(gd.V, gd.C, gd.bin_shift);
     }
     if (h->racc == reinterpret_cast<uint32_t *>(h->d_entries)) h->racc_zero = 0;  // entries take its place
@@ -3115,6 +3179,7 @@ int gz_server_admit(gz_server_t *s, uint32_t num_vertices, uint64_t seed, uint32
   gd.sketch_words = (gd.C * gd.B + 1) * 3;
   const size_t budget = tile_budget(&s->ingest, kServeTileC);
   MB_TRY(choose_tiles(gd, 0, budget, plane_fits(gd)));
+  gd.chosen = gd.plane;
   t.bytes = graph_sketch_bytes(gd);
   uint64_t off = 0;
   if (s->used + t.bytes > s->budget || !s->arena_alloc.alloc(t.bytes, off))
@@ -3248,12 +3313,14 @@ int gz_server_ingest(gz_server_t *s, uint32_t n, const uint32_t *ids, const void
   e->graphs.resize(n);
   for (uint32_t i = 0; i < n; ++i) e->graphs[i] = s->tenants[ids[i]].desc;
   e->d_flip = s->d_flip;
+  std::vector<uint64_t> rel(n + 1);
+  for (uint32_t i = 0; i <= n; ++i) rel[i] = offsets[i] - offsets[0];
+  bool retiled = false;
+  MB_TRY(choose_forms(e, rel.data(), call_sketch_bytes(e, rel.data()), &retiled));
   MB_TRY(finalize_graphs(e));
   MB_TRY(grow(&s->d_rec, s->rec_cap, nrec * 9, s->ingest.stream));
   MB_CUDA(cudaMemcpyAsync(s->d_rec, static_cast<const uint8_t *>(records) + offsets[0] * 9, nrec * 9,
                           cudaMemcpyHostToDevice, e->stream));
-  std::vector<uint64_t> rel(n + 1);
-  for (uint32_t i = 0; i <= n; ++i) rel[i] = offsets[i] - offsets[0];
   return batch_ingest(e, s->d_rec, rel.data());
 }
 
@@ -3283,6 +3350,8 @@ int gz_server_ingest_segments(gz_server_t *s, uint32_t nseg, const uint32_t *ten
   e->graphs.resize(ids.size());
   for (size_t i = 0; i < ids.size(); ++i) e->graphs[i] = s->tenants[ids[i]].desc;
   e->d_flip = s->d_flip;
+  bool retiled = false;
+  MB_TRY(choose_forms(e, off.data(), call_sketch_bytes(e, off.data()), &retiled));
   MB_TRY(finalize_graphs(e));
   MB_TRY(grow(&s->d_rec, s->rec_cap, nrec * 9, s->ingest.stream));
   uint64_t pos = 0;

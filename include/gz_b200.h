@@ -367,15 +367,19 @@ GZ_API int gz_batch_load_sketches(gz_batch_t *batch, uint32_t graph, const void 
  * CTAs sharing one SM (1..4, threads * CTAs <= 2048; each CTA stages its tiles in 1/ctas of the
  * SM's shared memory, so one CTA's bulk copies overlap another's XORs), and vertices per tile per
  * graph (NULL or 0 = the largest power of two <= 64 that fits). 0 picks the default (1024, 1), with which
- * graphs of at most 31 columns and no vertices per tile asked for are applied through bucket planes.
+ * graphs of at most 31 columns and no vertices per tile asked for are applied through bucket planes, or
+ * through staged tiles in calls of small graphs (up to 512 vertices) with few entries a vertex; the tiling
+ * that gz_batch_get_params gives is the last call's.
  * Sketch contents are kept; only the tiling changes. */
 GZ_API int gz_batch_set_tuning(gz_batch_t *batch, uint32_t threads_per_block, uint32_t ctas_per_sm,
                                const uint32_t *vertices_per_tile);
-/* Routing of each ingest call, per graph: a graph whose call brings few records for its size
- * (the in-place cost estimate, 2 (C + 1) bucket sectors per record, below sparse_factor times
- * the staged cost, its sketches read and written once plus the gutter's bytes) skips the
- * gutter: each record is hashed once and XORed into both endpoints' sketches in HBM. The rest
- * are guttered and applied tile by tile in shared memory. 0 = always staged, 1 = the default,
+/* Routing of each ingest call, per graph: a graph whose call brings few records for its size skips the
+ * gutter: each record is hashed once and XORed into both endpoints' sketches in HBM. The rest are
+ * guttered and applied tile by tile in shared memory. Where the engine chooses the form (no tile size
+ * or CTA shape asked for), few is sparse_factor times 36 entries a vertex while the call's graphs' sketches
+ * lie in L2, 2.5 past 1 GB of them (4 for graphs of at most 128 vertices), 4 between; where tiles are asked
+ * for, an in-place cost estimate, 2 (C + 1) bucket sectors per record, below sparse_factor times the staged
+ * cost, its sketches read and written once plus the gutter's bytes. 0 = always staged, 1 = the default,
  * a huge value = always in place. */
 GZ_API int gz_batch_set_route(gz_batch_t *batch, double sparse_factor);
 /* Autotuner: times trial ingests (records_per_vertex random edge records per vertex, 0 = 64) on
