@@ -1952,13 +1952,17 @@ int batch_flush_status(gz_batch *h) {
 //   2.5  more than 1 GB, graphs past 128 vertices: a record in place is then 1.3 ns of L2 reductions, a vertex
 //        through planes 1.3 ns (1e6 vertices in graphs of 1024: 2 entries 1.29 ms in place, 3.9 2.29, any
 //        through planes about 1.33);
-//   4    otherwise (1.5e5 vertices in graphs of 1024: 3.9 entries 0.26 ms in place, 0.27 through planes).
+//   4    otherwise (1.5e5 vertices in graphs of 1024: 3.9 entries 0.26 ms in place, 0.27 through planes);
+//   320 over the vertices, 36 at most, where that is more: the few sketches of a tiny graph stay in the cache
+//        while its records pass (1e6 vertices, staged against in place, ms: graphs of 16, 16 entries 2.89 and
+//        2.22; of 32, 8 entries 1.76 and 1.44, 16 1.82 and 2.48; of 64, 4 entries 1.72 and 1.33, 8 1.48 and 2.36).
 // Staged tiles asked for: staging the touched tiles moves about 2 x V x sketch bytes over HBM plus the gutter's
 // bytes, in place takes about 2 (C + 1) bucket sectors of 64 B per record.
 constexpr uint64_t kMbResidentBytes = 1ull << 27, kMbWideBytes = 1ull << 30;
 bool route_sparse(const gz_batch *h, const GraphDesc &gd, uint64_t n, uint64_t call_bytes) {
   if (gd.chosen) {
-    const double line = call_bytes <= kMbResidentBytes ? 36.0 : call_bytes > kMbWideBytes && gd.V > 128 ? 2.5 : 4.0;
+    const double far = std::max(call_bytes > kMbWideBytes && gd.V > 128 ? 2.5 : 4.0, std::min(36.0, 320.0 / gd.V));
+    const double line = call_bytes <= kMbResidentBytes ? 36.0 : far;
     return 2.0 * (double)n < line * gd.V * h->sparse_factor;
   }
   const double staged = 2.0 * gd.V * (gd.sketch_words * 4.0) + 50.0 * n;

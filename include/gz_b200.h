@@ -377,7 +377,8 @@ GZ_API int gz_batch_set_tuning(gz_batch_t *batch, uint32_t threads_per_block, ui
  * gutter: each record is hashed once and XORed into both endpoints' sketches in HBM. The rest are
  * guttered and applied tile by tile in shared memory. Where the engine chooses the form (no tile size
  * or CTA shape asked for), few is sparse_factor times 36 entries a vertex while the call's graphs' sketches
- * lie in L2, 2.5 past 1 GB of them (4 for graphs of at most 128 vertices), 4 between; where tiles are asked
+ * lie in L2, 2.5 past 1 GB of them (4 for graphs of at most 128 vertices), 4 between, and never less than
+ * 320 over the graph's vertices (36 at most); where tiles are asked
  * for, an in-place cost estimate, 2 (C + 1) bucket sectors per record, below sparse_factor times the staged
  * cost, its sketches read and written once plus the gutter's bytes. 0 = always staged, 1 = the default,
  * a huge value = always in place. */

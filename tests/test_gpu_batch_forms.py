@@ -78,3 +78,20 @@ def test_asked_tiles_stay(gz):
         before = _tiles(b)
         b.ingest([rec] * 700)
         assert _tiles(b) == before
+
+
+@pytest.mark.parametrize("V,entries,direct", [(16, 16, True), (16, 24, False), (32, 9, True), (32, 11, False),
+                                              (64, 4, True), (64, 6, False), (100, 3, True), (100, 5, False)])
+def test_records_of_tiny_graphs_go_in_place(gz, V, entries, direct):
+    """One kernel for records in place, several for the gutter and its tiles."""
+    G = (300 << 20) // (V * 2604)  # more than L2 holds, less than 1 GB
+    rec = _records(V, V * entries // 2, V)
+    with gz.CCSketchBatch([V] * G, [7] * G) as b:
+        b.ingest([rec] * G)
+        at = b.get_profile()["kernel_launches"]
+        b.ingest([rec] * G)
+        assert (b.get_profile()["kernel_launches"] - at == 1) == direct
+        b.ingest([rec] * G)
+        with gz.CCSketchAlg(V, 7) as a:
+            a.ingest_records(rec)
+            assert b.dump_sketches(G - 1).tobytes() == a.dump_sketches().tobytes()
