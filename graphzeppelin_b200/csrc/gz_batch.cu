@@ -2752,13 +2752,22 @@ int gz_batch_autotune(gz_batch_t *h, uint32_t records_per_vertex, uint32_t *vpt_
   }
   const uint32_t K = (uint32_t)keys.size();
   // scratch graphs: copies of each class's largest graph, enough (>= 16384 vertices, i.e. >= 4
-  // tiles per SM at 16 vertices per tile) that a class's trial fills the GPU like the real batch
-  std::vector<uint32_t> sv, first(K + 1, 0);
+  // tiles per SM at 16 vertices per tile) that a class's trial fills the GPU like the real batch, and as
+  // many sketches as the real batch has up to 1 GB (what a call costs beyond its tiles, and the route of
+  // its records, depend on it)
+  std::vector<uint32_t> sv, first(K + 1, 0), copies(K);
   std::vector<uint64_t> seeds;
+  uint64_t real_bytes = 0, scratch_bytes = 0;
+  for (const GraphDesc &gd : h->graphs) real_bytes += (uint64_t)gd.V * gd.sketch_words * 4;
   for (uint32_t k = 0; k < K; ++k) {
-    const uint32_t copies = std::max<uint32_t>(1, std::min<uint32_t>(64, (16384 + rep_v[k] - 1) / rep_v[k]));
+    copies[k] = std::max<uint32_t>(1, std::min<uint32_t>(64, (16384 + rep_v[k] - 1) / rep_v[k]));
+    scratch_bytes += (uint64_t)copies[k] * rep_v[k] * (keys[k].first * keys[k].second + 1) * 12;
+  }
+  const uint64_t want = std::min(real_bytes, kMbWideBytes);
+  const uint32_t times = (uint32_t)std::max<uint64_t>(1, (want + scratch_bytes - 1) / scratch_bytes);
+  for (uint32_t k = 0; k < K; ++k) {
     first[k] = (uint32_t)sv.size();
-    for (uint32_t c = 0; c < copies; ++c) {
+    for (uint32_t c = 0; c < copies[k] * times; ++c) {
       sv.push_back(rep_v[k]);
       seeds.push_back(0x5EEDull + sv.size());
     }
@@ -2791,6 +2800,17 @@ int gz_batch_autotune(gz_batch_t *h, uint32_t records_per_vertex, uint32_t *vpt_
   MB_CUDA(cudaGetLastError());
   MB_CUDA(cudaStreamSynchronize(sc->stream));
 
+  // device time of the whole ingest call, gutter and sketch update, at the scratch batch's tuning
+  auto trial = [&](const std::vector<uint64_t> &o, double *ms) -> int {
+    *ms = 1e300;
+    for (int rep = 0; rep < 3; ++rep) {
+      gz_batch_set_profiling(sc, 1);
+      MB_TRY(gz_batch_ingest_device(sc, guard.rec, o.data()));
+      if (rep) *ms = std::min(*ms, sc->prof_gutter_ms + sc->prof_sketch_ms);
+    }
+    return gz_batch_set_profiling(sc, 0);
+  };
+
   struct Shape {
     uint32_t threads, ctas;
   };
@@ -2810,12 +2830,8 @@ int gz_batch_autotune(gz_batch_t *h, uint32_t records_per_vertex, uint32_t *vpt_
         std::vector<uint32_t> vv(S, 0);
         for (uint32_t g = first[k]; g < first[k + 1]; ++g) vv[g] = vpt;
         if (gz_batch_set_tuning(sc, sh.threads, sh.ctas, vv.data()) != GZ_OK) continue;
-        double t = 1e300;
-        for (int rep = 0; rep < 3; ++rep) {
-          gz_batch_set_profiling(sc, 1);
-          MB_TRY(gz_batch_ingest_device(sc, guard.rec, o.data()));
-          if (rep) t = std::min(t, sc->prof_sketch_ms);
-        }
+        double t = 0;
+        MB_TRY(trial(o, &t));
         if (t < best) {
           best = t;
           pick[k] = vpt;
@@ -2830,22 +2846,17 @@ int gz_batch_autotune(gz_batch_t *h, uint32_t records_per_vertex, uint32_t *vpt_
       best_vpt = pick;
     }
   }
-  // the default form (bucket planes where they fit), timed the same way
-  double planes_total = 0;
+  // the default form (bucket planes where they fit) against the best staged one, all classes together: the
+  // choice of coded or plain entries is the batch's, and each form hashes in a different part of the call
+  std::vector<uint32_t> vv(S, 0);
+  for (uint32_t k = 0; k < K; ++k)
+    for (uint32_t g = first[k]; g < first[k + 1]; ++g) vv[g] = best_vpt[k];
+  double staged_ms = 0, planes_ms = 0;
+  MB_TRY(gz_batch_set_tuning(sc, best_shape.threads, best_shape.ctas, vv.data()));
+  MB_TRY(trial(off, &staged_ms));
   MB_TRY(gz_batch_set_tuning(sc, 0, 0, nullptr));
-  for (uint32_t k = 0; k < K; ++k) {
-    std::vector<uint64_t> o(S + 1);
-    for (uint32_t g = 0; g <= S; ++g) o[g] = std::min(std::max(off[g], off[first[k]]), off[first[k + 1]]);
-    double t = 1e300;
-    for (int rep = 0; rep < 3; ++rep) {
-      gz_batch_set_profiling(sc, 1);
-      MB_TRY(gz_batch_ingest_device(sc, guard.rec, o.data()));
-      if (rep) t = std::min(t, sc->prof_sketch_ms);
-    }
-    planes_total += t;
-  }
-  gz_batch_set_profiling(sc, 0);
-  if (planes_total <= best_total) {
+  MB_TRY(trial(off, &planes_ms));
+  if (planes_ms <= staged_ms) {
     MB_TRY(gz_batch_set_tuning(h, 0, 0, nullptr));
     for (uint32_t g = 0; vpt_out && g < h->G; ++g) vpt_out[g] = 1u << h->graphs[g].tile_shift;
     return GZ_OK;
