@@ -666,7 +666,7 @@ k_mb_plane_update(const GraphDesc *__restrict__ graphs, const uint32_t *__restri
     if (vg < V && lane < x.nc) {
       // what the write-back touches first is brought to L2 while the other warps finish
       asm volatile("prefetch.global.L2 [%0];" ::"l"(sk + 3 * lane * g.B));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(sk + 3 * lane * g.B + 16));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(sk + 3 * lane * g.B + column_second_word(g.B)));
     }
     __syncthreads();
     if (vg < V)

@@ -254,7 +254,7 @@ k_plane_update(const __grid_constant__ PlaneGeom g, const __grid_constant__ Hash
         if (c2 < C && (t2 << g.tile_shift) + vl < g.V) {
           const uint32_t *p = x.gsk + (uint64_t)((t2 << g.tile_shift) + vl) * g.sketch_words + 3 * c2 * B;
           asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 16));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p + column_second_word(B)));
         }
     }
     if (total == 0) continue;

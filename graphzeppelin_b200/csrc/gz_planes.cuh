@@ -34,6 +34,7 @@
 #include "gz_common.cuh"
 #include "gz_device.cuh"
 #include "gz_kernels.cuh"
+#include "gz_plane_layout.h"
 
 namespace gz {
 namespace dev {
