@@ -454,7 +454,7 @@ def run_b200(args, cfg):
                        "components": cfg["components"], "num_columns": p.num_columns,
                        "bkt_per_col": p.bkt_per_col, "sketch_bytes_total": V * p.sketch_bytes,
                        "entry_form": "coded (each record hashed once), bucket planes"
-                       if p.entry_form == 2 else "plain (hashed per endpoint), staged tiles",
+                       if p.entry_form == 2 else "plain (hashed per endpoint), bucket planes",
                        "stream_seed": cfg["stream_seed"], "sketch_seed": cfg["sketch_seed"],
                        "l2": "inputs larger than L2: 1.26 GB records + 1.29 GB sketches per step",
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},

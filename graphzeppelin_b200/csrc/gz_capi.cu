@@ -356,12 +356,9 @@ bool want_pipe(const gz_alg *h) {
 
 // Coded entries and bucket planes by default: CameoSketch of at most 31 columns up to 2^18
 // vertices (asked for explicitly: while the gutter bins fit the shared-memory hash sort). By
-// default a gutter bin is one tile of 32 vertices. Coarser bins (set_tuning tiles_per_bin 2..8)
-// lengthen the sort's runs but make every tile filter its bin's entries; measured on B200 over
-// 1.4e8 records at 2^17 vertices, gutter + sketch update took 5.2 + 6.4 ms at 1 tile per bin,
-// 5.0 + 7.1 ms at 2 and 4.8 + 8.0 ms at 4.
-constexpr uint32_t kPlaneBinTarget = 1024;
-constexpr uint32_t kPlaneTilesPerBin = 1;
+// default a gutter bin is one tile. Coarser bins (set_tuning tiles_per_bin 2..8) lengthen the sort's
+// runs but make every tile filter its bin's entries; over 1.4e8 records at 2^17 vertices in tiles of
+// 32, gutter + sketch update took 5.4 + 3.2 ms at 1 tile per bin, 5.3 + 5.0 at 2 and 4.8 + 6.6 at 4.
 constexpr uint32_t kPlaneDefaultMaxV = 1u << 18;
 
 int choose_planes(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tpb_req, bool &done) {
@@ -388,9 +385,6 @@ int choose_planes(gz_alg *h, uint32_t vpt_req, uint32_t threads_req, uint32_t tp
   if (tpb_req) {
     bshift = shift + (uint32_t)__builtin_ctz(tpb_req);
   } else {
-    while (((h->V + (1u << bshift) - 1) >> bshift) > kPlaneBinTarget &&
-           (1u << (bshift - shift)) < kPlaneTilesPerBin)
-      ++bshift;
     // large graphs: bins of several tiles, as many as the hash sort's shared memory holds
     while (((h->V + (1u << bshift) - 1) >> bshift) > gz::kSortBinsMax && bshift < shift + 3) ++bshift;
   }
@@ -645,7 +639,7 @@ int apply_pending(gz_alg *h) {
     const int per_sm = gz::plane_update_ctas_per_sm(h->tile_shift, (int)h->threads);
     const int grid = (int)std::min<uint64_t>(h->ntiles, (uint64_t)gz::num_sms() * per_sm);
     GZ_CUDA(gz::plane_update(h->pgeom(), h->ph, h->d_sk, h->d_gutter, h->chunks, h->d_bin_off,
-                             h->nchunks, h->d_status + 1, h->d_status, grid, (int)h->threads, h->stream));
+                             h->nchunks, h->d_status + 1, grid, (int)h->threads, h->stream));
   } else if (h->plain_planes) {
     GZ_CUDA(gz::plane_update_plain(h->pgeom(), h->cube, h->phw, h->d_sk, h->d_gutter, h->chunks, h->d_bin_off,
                                    h->nchunks, h->d_status + 1, h->stream));

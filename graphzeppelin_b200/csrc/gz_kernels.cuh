@@ -147,8 +147,7 @@ size_t plane_update_smem(uint32_t tile_shift, int threads);
 int plane_update_ctas_per_sm(uint32_t tile_shift, int threads);
 cudaError_t plane_update(const PlaneGeom &g, const PlaneHash &ph, uint8_t *sketches,
                          const uint8_t *gutter, const ChunkTable &chunks, const uint32_t *bin_off,
-                         int nchunks, uint32_t *work_counter, uint32_t *status, int grid,
-                         int threads, cudaStream_t s);
+                         int nchunks, uint32_t *work_counter, int grid, int threads, cudaStream_t s);
 // The same for plain entries, hashed where they are applied (any number of columns up to
 // kPlaneMaxColumnsWide, CameoSketch or CubeSketch), plane_threads(tile_shift) threads a CTA.
 int plane_threads(uint32_t tile_shift);

@@ -454,8 +454,7 @@ int plane_update_ctas_per_sm(uint32_t tile_shift, int threads) {
 
 cudaError_t plane_update(const PlaneGeom &g, const PlaneHash &ph, uint8_t *sketches,
                          const uint8_t *gutter, const ChunkTable &chunks, const uint32_t *bin_off,
-                         int nchunks, uint32_t *work_counter, uint32_t * /*status*/, int grid,
-                         int threads, cudaStream_t s) {
+                         int nchunks, uint32_t *work_counter, int grid, int threads, cudaStream_t s) {
   if (g.C > kPlaneMaxColumns || g.C < 18 || g.groups != 1 || g.tile_shift > 5 ||
       g.bin_shift < g.tile_shift || threads % 32 || threads < 32 || threads > 1024)
     return cudaErrorInvalidValue;
