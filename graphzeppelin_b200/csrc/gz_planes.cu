@@ -1,4 +1,5 @@
-// gz_planes.cu -- coded-entry record ingest for CameoSketch sketches of at most 31 columns.
+// gz_planes.cu -- record ingest through bucket planes: coded entries (CameoSketch of at most 31 columns),
+// plain entries (CubeSketch, more columns, large graphs), and records XORed straight into the sketches.
 //
 // Sketch::update (src/sketch.cpp:69-83) XORs an edge index and its checksum into the
 // deterministic bucket and into bucket (c, depth_c(idx)) of every column c, and
@@ -13,7 +14,9 @@
 //   k_plane_update       per tile of W vertices: the tile's entries (filtered out of their gutter
 //                        bin when a bin holds several tiles) XORed into bucket planes in shared
 //                        memory that start at zero, then each vertex's rows XORed into its sketch
-//                        in HBM. The checksum is hashed here, per entry.
+//                        in HBM. The checksum is hashed here, per entry (of a plain entry, the
+//                        columns too).
+//   k_direct_records     few records: each by a warp into both endpoints' sketches in HBM.
 // A coded entry is 128 bits: the C codes in bits 0 .. 4C - 1 (column c in bits 4c .. 4c + 3),
 // then the neighbour shifted left by bin_shift bits OR the vertex's offset inside its gutter bin
 // (the bin is known from where the entry lies). It is used when 4C + bin_shift + the neighbour's

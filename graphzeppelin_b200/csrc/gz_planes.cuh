@@ -7,18 +7,19 @@
 // plane row holds 32 slots, so slot s is shared-memory bank s and the 32 lanes of a step hit 32
 // different banks whatever their vertices and depths: the red.shared.xor never conflict (the
 // per-entry ordering, every lane on column c at once, concentrates lanes on a few banks because
-// depth 0 takes half the updates). Each bucket is kept as three words,
+// depth 0 takes half the updates). Each bucket is kept as four words,
 //   A = XOR of (neighbour | 1 << 31) over the entries whose neighbour is above the vertex,
-//   B = the same over the other entries,
-//   G = XOR of their checksums,
-// so one update XORs two words (A or B, and G) instead of three. With idx = (min << 32) | max
+//   GA = XOR of their checksums,
+//   B and GB = the same over the other entries (the bucket's gamma is GA ^ GB),
+// so one update XORs two words (A and GA, or B and GB) instead of three. With idx = (min << 32) | max
 // (concat_pairing_fn, src/util.cpp:45-51) the bucket's alpha is recovered as
 //   alpha low  = low31(A) ^ (top bit of B ? vertex : 0),
 //   alpha high = low31(B) ^ (top bit of A ? vertex : 0),
 // the top bits holding the parity of each kind's entry count (vertex ids are below 2^31).
 // Rows hold depths 0 .. kPlaneRows - 2; the last row collects the depths at or above it (2^-11 of
-// the column updates), which are XORed into the sketch in HBM with global atomics; those rows are
-// never touched by the write-back, which changes only the rows the planes hold.
+// the column updates), which are XORed into the sketch in HBM with global atomics; the write-back changes
+// only the buckets of the rows above it (CubeSketch, whose buckets take every depth from their own on,
+// counts the last row in).
 //
 // What bounds the update: shared-memory issue. A slot step is two red.shared.xor, one wavefront
 // each, 64 wavefronts per 32 entries and SM. The address of a step is made by one byte permute

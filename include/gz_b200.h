@@ -81,8 +81,10 @@ typedef struct gz_params {
   uint32_t sketch_algorithm;    /* enum gz_sketch_algorithm */
   uint32_t in_place;            /* 1: sketches too large to stage in shared memory are updated in HBM */
   uint32_t entry_form;          /* gutter entries of records: 1 = plain (hashed per endpoint where
-                                   applied), 2 = coded (each record hashed once, bucket planes),
-                                   3 = coded with 3-bit depth codes (larger graphs) */
+                                   applied: bucket planes in a handle left to itself, staged tiles
+                                   where gz_set_tuning or gz_set_pipeline asked for a form), 2 = coded
+                                   (each record hashed once, bucket planes), 3 = coded with 3-bit
+                                   depth codes (larger graphs) */
 } gz_params_t;
 
 /* One sampled component of one Boruvka round (parity tracing). key = smallest member id. */
@@ -295,18 +297,20 @@ GZ_API int gz_measure_update_rate(int repeats, double *updates_per_s);
 /* Tuning knobs of the ingest kernels (0 picks the default): vertices per shared-memory tile
  * (power of two in [4, 64]; at most 32 with coded entries), threads per block of the
  * sketch-update kernel, tiles per gutter bin (power of two <= 64; 1 with coded entries), and the
- * gutter entry form for records: 1 = plain entries {vertex, neighbour} (hashed per endpoint by the
- * sketch update), 2 = coded entries (each record hashed once in the gutter into
+ * gutter entry form for records: 1 = plain entries {vertex, neighbour} (hashed per endpoint by a
+ * staged-tile sketch update), 2 = coded entries (each record hashed once in the gutter into
  * per-column depth codes, applied through bucket planes; CameoSketch with at most 31 columns and
  * at most 8192 gutter bins; 4-bit codes where they fit a 16-byte entry, else 3-bit codes),
  * 3 = coded entries with 3-bit codes (code 7 = depth 7 or more, hashed again where applied).
- * 0 picks coded entries where they apply. Buffered updates are applied first. */
+ * 0 picks coded entries up to 2^18 vertices where they apply; with every other knob at 0 too, plain
+ * entries through bucket planes elsewhere. Buffered updates are applied first. */
 GZ_API int gz_set_tuning(gz_alg_t *alg, uint32_t vertices_per_tile, uint32_t threads_per_block,
                          uint32_t tiles_per_bin, uint32_t entry_form);
-/* Route of sparse tiles (one tile per gutter bin, plain CameoSketch entries): a tile holding
- * fewer entries than factor x (its sketch bytes / (32 (columns + 1))) -- the break-even of
- * staging it in shared memory against updating its buckets in HBM -- is updated in place with
- * global atomics. 0 = always staged, 1 = the default. Same role as gz_batch_set_route. */
+/* Route of few updates (CameoSketch): a tile holding fewer entries than factor x its break-even --
+ * staging it, or writing its bucket planes back, against updating its buckets in HBM -- is updated in
+ * place with global atomics, and records that arrive between two flushes and are fewer than that
+ * for the whole graph skip the gutter. 0 = always the gutter and its tiles, 1 = the default. Same role
+ * as gz_batch_set_route. */
 GZ_API int gz_set_direct_factor(gz_alg_t *alg, double factor);
 /* How queries run. mode = 2: the whole Boruvka emulation in one kernel launch, every round on the
  * device with barriers over the launch between its phases (one thread-block cluster for small
