@@ -2633,6 +2633,7 @@ int gz_batch_destroy(gz_batch_t *h) {
 
 int gz_batch_get_params(gz_batch_t *h, uint32_t graph, gz_params_t *o) {
   if (!h || !o || graph >= h->G) return mb_fail(GZ_ERR_INVALID, "bad argument");
+  std::lock_guard<std::mutex> lk(h->mtx);  // an ingest call may tile the graph anew
   const GraphDesc &gd = h->graphs[graph];
   std::memset(o, 0, sizeof(*o));
   o->num_vertices = gd.V;

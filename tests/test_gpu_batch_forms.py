@@ -95,3 +95,33 @@ def test_records_of_tiny_graphs_go_in_place(gz, V, entries, direct):
         with gz.CCSketchAlg(V, 7) as a:
             a.ingest_records(rec)
             assert b.dump_sketches(G - 1).tobytes() == a.dump_sketches().tobytes()
+
+
+def test_params_while_another_thread_ingests(gz):
+    """The tiling is read whole while calls of other densities change it."""
+    import threading
+    V, G = 256, 300
+    few, many = _records(V, 8 * V // 2, 1), _records(V, 60 * V // 2, 2)
+    with gz.CCSketchBatch([V] * G, [7] * G) as b:
+        b.set_route(0.0)
+        done = threading.Event()
+        seen, errors = set(), []
+
+        def read():
+            try:
+                while not done.is_set():
+                    b._refresh_params()
+                    p = b.params[G // 2]
+                    seen.add((p.vertices_per_tile, p.num_tiles, p.vertices_per_bin, p.num_bins))
+            except BaseException as e:  # noqa: BLE001
+                errors.append(e)
+
+        t = threading.Thread(target=read)
+        t.start()
+        for _ in range(20):
+            b.ingest([few] * G)
+            b.ingest([many] * G)
+        done.set()
+        t.join(60)
+        assert not errors and not t.is_alive()
+        assert seen <= {(8, 32, 8, 32), (32, 8, 32, 8)}
