@@ -2253,11 +2253,12 @@ int enqueue_round(gz_batch *h, cudaStream_t s) {
 // and 2.5 ms, 2.05e6 2.8 and 4.3, 4.1e6 5.4 and 7.7, 8.2e6 10.8 and 14.7.
 // The accumulators take about 350 to 500 B a vertex. Where the gutter's entry buffer, idle between
 // ingests, is large enough they lie there, and are cleared by the first query after an ingest. Otherwise the
-// handle's first block comes from cudaMalloc when it is large: the stream-ordered pool grew by 512 MB in 3.2
-// ms and by 2 GB in 12 to 51, cudaMalloc gives them in 0.6 to 1.7 and 0.7 to 3.5. A block that is outgrown goes
-// on from the pool, whose regrowth does not wait for the device. (A process's first query, graphs of 1024
-// vertices with 6,000 records each: 2.05e6 vertices 7.6 -> 4.6 ms, 8.2e6 27 -> 13.3, with 600 records each 28
-// -> 14; in rounds 5.7, 16.7 and 17.4.)
+// first block of a batch of its own comes from cudaMalloc when it is large: the stream-ordered pool grew by 512
+// MB in 3.2 ms and by 2 GB in 12 to 51, cudaMalloc gives them in 0.6 to 1.7 and 0.7 to 3.5. (A batch's graphs do
+// not change, so the block is not outgrown; a server's queries vary, and its engine stays with the pool, whose
+// regrowth does not wait for the device.) A process's first query, graphs of 1024 vertices with 6,000 records
+// each: 2.05e6 vertices 7.6 -> 4.6 ms, 8.2e6 27 -> 13.3, with 600 records each 28 -> 14; in rounds 5.7, 16.7
+// and 17.4.
 constexpr uint64_t kMbOneLaunchMaxV = 1u << 23;
 constexpr uint32_t kQresCtl = 8;  // go, barrier
 constexpr uint64_t kQbufPlainWords = 1ull << 24;  // 64 MB
@@ -2267,7 +2268,7 @@ uint64_t vstate_at(const gz_batch *h, uint64_t cap) { return (cap - (6 * h->tota
 int grow_qbuf(gz_batch *h, uint64_t words) {
   if (h->d_qbuf && h->cap_qbuf >= words) return GZ_OK;
   const uint64_t n = headroom(h->cap_qbuf, words);
-  const bool plain = !h->d_qbuf && n >= kQbufPlainWords;
+  const bool plain = h->own_storage && !h->d_qbuf && n >= kQbufPlainWords;
   h->cap_qbuf = h->racc_zero = 0;
   if (h->qbuf_plain) mb_free(h->d_qbuf);
   h->qbuf_plain = false;
