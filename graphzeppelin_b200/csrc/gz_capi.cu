@@ -177,7 +177,6 @@ struct gz_alg {
   gz::BoruvkaBufs bv{};
   bool bv_alloc = false;
   uint32_t *d_final = nullptr, *d_ncc = nullptr;
-  uint2 *d_edges = nullptr;  // the spanning forest's edges, on their way to the host
   uint32_t n_forest = 0;     // edges of the device answer's forest: one per union, V less its components
   bool dsu_valid = true, update_locked = false, labels_on_host = false;
   // eager DSU (the reference's default build, src/cc_sketch_alg.cpp:87-102): a host union-find
@@ -588,7 +587,6 @@ void destroy_alg(gz_alg *h) {
   }
   dev_free(h->d_raw);
   free_bv(h->bv);
-  dev_free(h->d_edges);
   for (auto &e : h->prof_pending) {
     cudaEventDestroy(e.a);
     cudaEventDestroy(e.b);
@@ -858,9 +856,10 @@ int forest_to_host(gz_alg *h, uint32_t *edges_out, size_t cap, size_t *n_edges) 
   *n_edges = h->n_forest;
   const size_t n = std::min<size_t>(cap, h->n_forest);
   if (!edges_out || !n) return GZ_OK;
-  GZ_TRY(dev_alloc(&h->d_edges, h->V));
-  GZ_CUDA(gz::forest_edges(h->bv, h->V, h->d_edges, h->stream));
-  GZ_CUDA(cudaMemcpyAsync(edges_out, h->d_edges, n * sizeof(uint2), cudaMemcpyDeviceToHost, h->stream));
+  // every query sets the labels and smallest members anew: their place holds V edges meanwhile
+  uint2 *edges = reinterpret_cast<uint2 *>(h->bv.label);
+  GZ_CUDA(gz::forest_edges(h->bv, h->V, edges, h->stream));
+  GZ_CUDA(cudaMemcpyAsync(edges_out, edges, n * sizeof(uint2), cudaMemcpyDeviceToHost, h->stream));
   GZ_CUDA(cudaStreamSynchronize(h->stream));
   return GZ_OK;
 }
@@ -910,8 +909,7 @@ int alloc_bv(gz::BoruvkaBufs &b, size_t V, uint32_t *status, uint32_t **labels, 
   if (b.block) return GZ_OK;
   Block k;
   k.take(&b.parent, V);
-  k.take(&b.label, V);
-  k.take(&b.minv, V);
+  k.take(&b.label, 2 * V);  // minv behind it: between queries, the forest's edges on their way to the host
   k.take(&b.forest, V);
   k.take(labels, V);
   k.take(&b.round, 8);  // round, ctl[3], components, forest edges
@@ -919,6 +917,7 @@ int alloc_bv(gz::BoruvkaBufs &b, size_t V, uint32_t *status, uint32_t **labels, 
   k.take(&b.forest_n, 1);
   k.take(&b.trace_n, 1);
   GZ_TRY(k.alloc(&b.block));
+  b.minv = b.label + V;
   b.ctl = b.round + 1;
   *ncc = b.round + 4;
   b.edge_n = b.round + 5;

@@ -69,3 +69,28 @@ def test_forest_bytes(gz, tmp_path):
     assert _copied(torch, tmp_path, lambda: a.lib.gz_spanning_forest(
         a._h, buf.ctypes.data, want // 4, ctypes.byref(n))) <= 8 * (want // 4) + 64
     a.close()
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_forest_takes_no_memory_and_queries_go_on(gz, mode):
+    """A fetch uses what the query left behind; later queries, traced or not, are as on a fresh handle."""
+    torch = pytest.importorskip("torch")
+    from graphzeppelin_b200 import streams as S
+    V = 1 << 18
+    a = _handle(gz, V, mode, 3)
+    a.num_connected_components()
+    rng = np.random.default_rng(3)
+    more = S.make_records(rng.integers(0, V, 9).astype(np.uint32), rng.integers(0, V, 9).astype(np.uint32))
+    before = torch.cuda.mem_get_info()[0]
+    a.calc_spanning_forest()
+    assert before - torch.cuda.mem_get_info()[0] < 1 << 20
+    b = _handle(gz, V, mode, 3)
+    for alg in (a, b):
+        alg.set_trace(True)
+        alg.ingest_records(more)
+    x, y = a.connected_components(), b.connected_components()
+    assert (x.parent_arr == y.parent_arr).all() and a.last_query_rounds == b.last_query_rounds
+    assert sorted(a.get_trace().tolist()) == sorted(b.get_trace().tolist())
+    assert len(a.calc_spanning_forest().get_edges()) == V - x.size()
+    a.close()
+    b.close()
