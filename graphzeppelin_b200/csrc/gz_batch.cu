@@ -1162,6 +1162,7 @@ struct MbQuery {
   uint32_t *rstate, *racc, *det;                     // per vertex: state, accumulator, deterministic bucket
   uint32_t *lastmod, *ncc, *go, *qbar, *labels;
   uint32_t sw, G;  // words of an accumulator; graphs
+  uint32_t clear;  // the accumulators may hold anything: round 0 clears each beside its vertex's sample
 };
 constexpr int kMbqMaxThreads = 768;
 // the ring's stage (its words + 3) also holds the 32 words of a warp's permutation
@@ -1308,6 +1309,10 @@ __global__ void __launch_bounds__(kMbqMaxThreads, 1) k_mb_query(MBBufs b, MbQuer
       if (lane < nm) {
         const uint32_t *d = reinterpret_cast<const uint32_t *>(ring.slot(T + t, lane, kMbKB) + ring.run_cap + (offs >> 8));
         reinterpret_cast<uint4 *>(q.det)[v0 + lane] = make_uint4(d[0], d[1], d[2], 0);
+      }
+      if (q.clear) {
+        uint4 *ac = reinterpret_cast<uint4 *>(q.racc + (uint64_t)v0 * SW);
+        for (uint32_t i = lane; i < nm * (SW / 4); i += 32) ac[i] = make_uint4(0, 0, 0, 0);
       }
       offs = offs_next;
       __syncwarp();
@@ -2252,7 +2257,8 @@ int enqueue_round(gz_batch *h, cudaStream_t s) {
 // batch_query_rounds then run. Graphs of 1024 vertices, launch against rounds: 1.02e6 vertices together 1.5
 // and 2.5 ms, 2.05e6 2.8 and 4.3, 4.1e6 5.4 and 7.7, 8.2e6 10.8 and 14.7.
 // The accumulators take about 350 to 500 B a vertex. Where the gutter's entry buffer, idle between
-// ingests, is large enough they lie there, and are cleared by the first query after an ingest. Otherwise the
+// ingests, is large enough they lie there, and the first query after an ingest clears them in its round 0 (128
+// graphs, 0.6 GB: a memset ahead of it took 0.1 ms of 14.9, beside the samples it is not seen). Otherwise the
 // first block of a batch of its own comes from cudaMalloc when it is large: the stream-ordered pool grew by 512
 // MB in 3.2 ms and by 2 GB in 12 to 51, cudaMalloc gives them in 0.6 to 1.7 and 0.7 to 3.5. (A batch's graphs do
 // not change, so the block is not outgrown; a server's queries vary, and its engine stays with the pool, whose
@@ -2345,8 +2351,7 @@ int batch_query_launch(gz_batch *h, uint32_t *labels_out, uint64_t *zero_after) 
   // a query that ran to its end leaves every accumulator zero
   const uint64_t zero = h->racc_zero;
   h->racc_zero = 0;
-  if (zero < racc_total)
-    MB_CUDA(cudaMemsetAsync(h->racc + zero, 0, sizeof(uint32_t) * (racc_total - zero), h->stream));
+  q.clear = zero < racc_total;
   *zero_after = std::min(std::max(zero, racc_total), states);
   MBBufs a_b = b;
   void *args[] = {&a_b, &q};
